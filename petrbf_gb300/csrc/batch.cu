@@ -280,7 +280,7 @@ void batch_interpolate(Ctx& c, int nprob, const prbf_problem* probs, int* its_ou
     // truncation-set sizes (the per-problem plan) and buffer-list sizes
     GaussPlan lp;
     lp.g = P.g;
-    gauss_plan_dev(lp, P.view(), P.view(), c.err.get(), c.ws, c.stream, false);
+    gauss_plan_dev(lp, P.view(), P.view(), c.err.get(), c.ws, c.stream, 0);
     PRBF_CUDA(cudaMemcpyAsync(B.trunc.get() + co, lp.trunc_cnt.get(), sizeof(int) * nc, cudaMemcpyDeviceToDevice,
                               c.stream));
     pairs += lp.pairs;
@@ -308,10 +308,9 @@ void batch_interpolate(Ctx& c, int nprob, const prbf_problem* probs, int* its_ou
   B.plan.cprob.reserve(NC);
   PRBF_CUDA(cudaMemcpyAsync(B.plan.grids.get(), hgrids.data(), sizeof(Grid) * nprob, cudaMemcpyHostToDevice, c.stream));
   PRBF_CUDA(cudaMemcpyAsync(B.plan.cprob.get(), B.cprob.get(), sizeof(int) * NC, cudaMemcpyDeviceToDevice, c.stream));
-  B.plan.f32_ready = false;
-  if (mixed)
-    gauss_plan_f32_batch(B.plan, hgrids,
-                         PointsView{N, B.x.get(), B.y.get(), dim == 3 ? B.z.get() : nullptr, B.cs.get()}, c.stream);
+  gauss_plan_forms_batch(B.plan, hgrids,
+                         PointsView{N, B.x.get(), B.y.get(), dim == 3 ? B.z.get() : nullptr, B.cs.get()},
+                         FORM_F64 | (mixed ? FORM_F32 : 0), c.stream);
 
   // ---- pass 2: buffer lists into the global block arrays, then one batched factorisation
   std::vector<long long> hb((size_t)NC + 1);

@@ -40,6 +40,7 @@ Grid make_grid(int dim, const double* b, double sigma, int nsigma_box, int sigma
   g.ncell = g.nx * g.ny * g.nz;
   g.trunc_len = sigma_trunc * sigma / 2 + kEpsf;
   g.buffer_len = sigma_buffer * sigma / 2 + kEpsf;
+  g.norm = 1.0 / (2 * 3.141592653589793 * sigma * sigma);
   return g;
 }
 
@@ -356,7 +357,7 @@ int prbf_evaluate(prbf_ctx* ctx, int nt, const double* xt, const double* yt, con
     gather_dev(ns, S.perm.get(), sg.get(), sgs.get(), c.stream);
     GaussPlan plan;
     plan.g = g;
-    gauss_plan_dev(plan, T.view(), S.view(), c.err.get(), c.ws, c.stream);
+    gauss_plan_dev(plan, T.view(), S.view(), c.err.get(), c.ws, c.stream, FORM_F64);
     w.reserve((size_t)nt + 4);
     PRBF_CUDA(cudaMemsetAsync(w.get(), 0, sizeof(double) * nt, c.stream));
     gauss_sum_dev(plan, T.view(), S.view(), sgs.get(), w.get(), false, c.err.get(), c.stream);

@@ -49,6 +49,7 @@ struct Grid {
   double box;               // nsigma_box*sigma + epsf
   double trunc_len;         // sigma_trunc*sigma/2 + epsf
   double buffer_len;        // sigma_buffer*sigma/2 + epsf
+  double norm;              // 1/(2 pi sigma^2)
 };
 
 // Work of stopped systems in a batch: cell -> problem, and the problems' stop flags

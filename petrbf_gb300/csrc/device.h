@@ -101,13 +101,19 @@ struct GaussPlan {
   DevBuf<Grid> grids;     // batched: one grid per problem (with its first global cell)
   DevBuf<int> cprob;      // batched: problem of each global cell
   SegSkip seg;            // batched: skip the items of stopped problems (when seg.done set)
-  // FP32 form: per-source FP32 cell-relative coordinates and truncation masks (built by
-  // gauss_plan_dev when nb_trunc <= 7 and ny < 65536), and a FP32 copy of <= 4 weight
-  // vectors at stride g32_stride
+  // FP32 form: per-source FP32 cell-relative coordinates and truncation masks (the masks
+  // serve the fixed-point form too; built when nb_trunc <= 7 and ny < 65536), and a FP32
+  // copy of <= 4 weight vectors at stride g32_stride
   bool f32_ready = false;
   long long g32_stride = 0;
   DevBuf<float> su, sv, sw, g32;
   DevBuf<unsigned long long> smask;
+  // FP64 form with fixed-point exponents (gauss_fx.cuh): the sources' coordinates, and the
+  // targets' where they are another point set
+  bool fx_ready = false;
+  bool fx_self = true;
+  int fx_ncs = 0;  // entries of the cell starts
+  DevBuf<uint2> fxs[3], fxt[3];
   // FP64 matvec with each exponential used for both rows (targets == sources, every cell
   // <= 128 points): K partial slots of pstride entries per weight vector, for up to sym_nv
   // vectors per launch (set sym_nv before gauss_plan_dev; kept zero between products), and
@@ -115,6 +121,7 @@ struct GaussPlan {
   bool sym_ready = false;
   int sym_nv = 1;
   int sym_K = 0;
+  int sym_sets = 1;  // slots per window cell (the fixed-point form: one per pass over a cell)
   long long sym_pstride = 0;
   DevBuf<double> sym_part;
   DevBuf<unsigned long long> sym_cy;
@@ -123,14 +130,18 @@ struct GaussPlan {
   DevBuf<int2> sym_items;
 };
 
-// Builds the work list and the truncation-set sizes; sets plan.pairs / max_trunc. forms:
-// also the FP32 form's source data and the symmetric FP64 form's buffers (a plan used only
-// for its sizes passes false).
+// The forms of the sum a plan is used for: the FP32 products, the FP64 products (neither for
+// a plan used only for its sizes).
+enum : int { FORM_F32 = 1, FORM_F64 = 2 };
+// Builds the work list and the truncation-set sizes; sets plan.pairs / max_trunc, and the
+// point data of the forms asked for.
 void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& src,
-                    unsigned* err, Workspace& ws, cudaStream_t s, bool forms = true);
-// FP32 form's source data of a batch (each problem with its own grid and scale, grids with
-// their first global cell); sets plan.f32_ready when every grid qualifies.
-void gauss_plan_f32_batch(GaussPlan& plan, const std::vector<Grid>& grids, const PointsView& src, cudaStream_t s);
+                    unsigned* err, Workspace& ws, cudaStream_t s, int forms = FORM_F32 | FORM_F64);
+// Point data of a batch (plan.grids and plan.cprob set: each problem with its own grid and
+// scale, grids with their first global cell); sets plan.f32_ready / fx_ready for the forms
+// asked for when every grid qualifies.
+void gauss_plan_forms_batch(GaussPlan& plan, const std::vector<Grid>& grids, const PointsView& src, int forms,
+                            cudaStream_t s);
 // Symmetric FP64 form of a batch (every grid with the same window, every cell <= 128
 // points; hcs: the global cell starts on the host); false when it does not apply.
 bool gauss_plan_sym_batch(GaussPlan& plan, const std::vector<Grid>& grids, const PointsView& src,

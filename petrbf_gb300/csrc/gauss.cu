@@ -17,10 +17,12 @@
 //      in order, into a second shared buffer (as cell-relative, scaled coordinates);
 //   3. each warp takes groups of kGroup targets, its lanes stride over the compacted
 //      sources, and the partial sums are reduced with warp shuffles.
-// FP64 form: exp on the FP64 pipe with a table-folded polynomial (12 FP64 instructions
-// per pair, range reduction bits and the 2^-m scaling on the integer pipe); coordinates
-// relative to the cell centre, unscaled, so x_t - x_s rounds as in the reference. FP32
-// form: scaled FP32 coordinates relative to the cell centre and the SFU exp2.
+// FP64 form: grids whose windows fit the fixed-point exponents of gauss_fx.cuh take the
+// kernels of gauss_fx.cu; the others (wider than 18 sigma, more than 15 cells across, beyond
+// 65535 cells in y) the kernels here, with exp on the FP64 pipe by a table-folded polynomial
+// (12 FP64 instructions per pair, range reduction bits and the 2^-m scaling on the integer
+// pipe); coordinates relative to the cell centre, unscaled, so x_t - x_s rounds as in the
+// reference. FP32 form: scaled FP32 coordinates relative to the cell centre and the SFU exp2.
 //
 // NV weight vectors (several right-hand sides of one point set, NV <= 4) are summed in
 // one pass: each pair's exponential is computed once and multiplies NV weights.
@@ -29,17 +31,14 @@
 #include <cmath>
 
 #include "device.h"
+#include "gauss_common.cuh"
+#include "gauss_fx.cuh"
 
 namespace prbf {
 namespace {
 
-constexpr int kThreads = 128;  // 4 warps
-constexpr int kWarps = kThreads / 32;
-constexpr int kTileT = 128;    // targets per work item
 constexpr int kGroup = 4;      // targets per warp pass
 constexpr int kRawCap = 1024;  // staged raw sources per fill (incl. alignment padding)
-constexpr int kMaxPieces = 64; // source ranges per fill
-constexpr int kMaxRanges = 256; // column ranges of an item kept in shared memory
 
 // exp table: e^a with a = -L*d, d >= 0, L = ln2/n:  k = rint(d), r = k - d in [-1/2, 1/2],
 // e^a = 2^(-k/n) e^(L r) = 2^-m T[j] p(r),  k = m*n + j; the table holds T[j] c_i
@@ -74,14 +73,6 @@ struct Cfg {
   static constexpr int kRaw = k3d64 ? 512 : kRawCap;
   using T = typename std::conditional<F32, float, double>::type;
 };
-
-struct Piece {
-  int raw_off;  // smem index of the first valid element
-  int count;    // valid elements
-  int gstart;   // global (sorted) index of the first valid element
-};
-
-constexpr size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
 
 // Dynamic shared memory carve-up of k_gauss (byte offsets, each 16-byte aligned).
 template <int DIM, bool F32, int NV>
@@ -436,33 +427,67 @@ __global__ void __launch_bounds__(kThreads, GaussMinBlocks<F32>::v) k_gauss(
 // as the FP64 kernel, so the truncation set is identical), and jy in the top 16 bits. The
 // per-source filter is then integer work and the target-relative coordinate is
 // u_j + (jx - ix) box scale, one FP32 add (the FP64 path rounds once from FP64 instead).
-constexpr int kMaskBits = 15;    // 2 nb + 1 <= 15 bits per axis: nb_trunc <= 7
-constexpr int kMaskY = kMaskBits, kMaskZ = 2 * kMaskBits, kMaskCellY = 48;
 constexpr int kAlignF = 4;       // elements per 16 bytes (FP32 arrays; the masks use 2 x 16)
 
-__global__ void k_src_f32(Grid g, const int* __restrict__ cs, const double* __restrict__ x,
-                          const double* __restrict__ y, const double* __restrict__ z, double scale,
-                          float* __restrict__ U, float* __restrict__ V, float* __restrict__ W,
-                          unsigned long long* __restrict__ M) {
-  const int nb = g.nb_trunc;
+// The FP64 form with fixed-point exponents (gauss_fx.cuh) takes the same words and fixed-
+// point coordinates instead.
+struct PointForms {  // null: not wanted
+  float *u = nullptr, *v = nullptr, *w = nullptr;
+  unsigned long long* mask = nullptr;
+  uint2 *fx = nullptr, *fy = nullptr, *fz = nullptr;
+};
+
+// A warp per cell (of one grid, or of a batch's: cell -> problem -> grid): its lanes stride
+// over the cell's points, the centres of the cells at offsets -nb .. nb computed once.
+// Bound by the FP64 pipe (the box tests): 4x10^6 points in 2D.
+__global__ void __launch_bounds__(256) k_point_forms(Grid g0, const Grid* __restrict__ grids,
+                                                     const int* __restrict__ cprob, int ncell,
+                                                     const int* __restrict__ cs, const double* __restrict__ x,
+                                                     const double* __restrict__ y, const double* __restrict__ z,
+                                                     PointForms o) {
+  __shared__ double s_ctr[8][3][kMaskBits];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c = blockIdx.x * 8 + wid;
+  if (c >= ncell) return;
+  const int a = cs[c], b = cs[c + 1];
+  if (a == b) return;
+  const Grid g = grids ? grids[cprob[c]] : g0;
+  const int nb = g.nb_trunc, W = 2 * nb + 1;
   const double L = g.trunc_len;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.ncell; c += gridDim.x * blockDim.x) {
-    int ix, iy, iz;
-    cell_xyz(g, c, ix, iy, iz);
-    const double xc = centre_coord(g.xmin, ix, g.box), yc = centre_coord(g.ymin, iy, g.box);
-    const double zc = g.dim == 3 ? centre_coord(g.zmin, iz, g.box) : 0.0;
-    for (int j = cs[c]; j < cs[c + 1]; j++) {
+  int ix, iy, iz;
+  cell_xyz(g, c - g.cbase, ix, iy, iz);
+  if (o.mask) {
+    for (int q = lane; q < W; q += 32) {  // bit q: the target cell at offset q - nb from this one
+      s_ctr[wid][0][q] = centre_coord(g.xmin, ix - (q - nb), g.box);
+      s_ctr[wid][1][q] = centre_coord(g.ymin, iy - (q - nb), g.box);
+      s_ctr[wid][2][q] = g.dim == 3 ? centre_coord(g.zmin, iz - (q - nb), g.box) : 0.0;
+    }
+    __syncwarp();
+  }
+  const double xc = centre_coord(g.xmin, ix, g.box), yc = centre_coord(g.ymin, iy, g.box);
+  const double zc = g.dim == 3 ? centre_coord(g.zmin, iz, g.box) : 0.0;
+  const double scale = o.u ? sum_consts(g.sigma, true, 0).scale : 0.0;
+  const FxScale fs = o.fx ? fx_scale(g.sigma) : FxScale{0.0, 0.0};
+  for (int j = a + lane; j < b; j += 32) {
+    const double px = x[j], py = y[j], pz = g.dim == 3 ? z[j] : 0.0;
+    if (o.mask) {
       unsigned long long m = (unsigned long long)iy << kMaskCellY;
-      for (int k = 0; k <= 2 * nb; k++) {
-        const int o = k - nb;  // source cell - target cell
-        if (fabs(x[j] - centre_coord(g.xmin, ix - o, g.box)) < L) m |= 1ull << k;
-        if (fabs(y[j] - centre_coord(g.ymin, iy - o, g.box)) < L) m |= 1ull << (kMaskY + k);
-        if (g.dim == 3 && fabs(z[j] - centre_coord(g.zmin, iz - o, g.box)) < L) m |= 1ull << (kMaskZ + k);
+      for (int q = 0; q < W; q++) {
+        if (fabs(px - s_ctr[wid][0][q]) < L) m |= 1ull << q;
+        if (fabs(py - s_ctr[wid][1][q]) < L) m |= 1ull << (kMaskY + q);
+        if (g.dim == 3 && fabs(pz - s_ctr[wid][2][q]) < L) m |= 1ull << (kMaskZ + q);
       }
-      U[j] = (float)((x[j] - xc) * scale);
-      V[j] = (float)((y[j] - yc) * scale);
-      if (g.dim == 3) W[j] = (float)((z[j] - zc) * scale);
-      M[j] = m;
+      o.mask[j] = m;
+    }
+    if (o.u) {
+      o.u[j] = (float)((px - xc) * scale);
+      o.v[j] = (float)((py - yc) * scale);
+      if (g.dim == 3) o.w[j] = (float)((pz - zc) * scale);
+    }
+    if (o.fx) {
+      o.fx[j] = fx_coord(px, fs.hi, fs.lo);
+      o.fy[j] = fx_coord(py, fs.hi, fs.lo);
+      if (g.dim == 3) o.fz[j] = fx_coord(pz, fs.hi, fs.lo);
     }
   }
 }
@@ -1482,6 +1507,12 @@ void launch_sym_k(const GaussPlan& P, const PointsView& s, const double* gv, dou
   PRBF_CHECK_LAUNCH();
 }
 
+void launch_sym_gather(const GaussPlan& P, int n, int nv, double* w, long long vs, const int* skip, cudaStream_t st) {
+  const int gb = std::max(1, std::min(ceil_div(n, 256), 8 * 152));
+  k_sym_gather<<<gb, 256, 0, st>>>(n, nv, P.sym_K * P.sym_sets, P.sym_pstride, P.sym_part.get(), w, vs, skip);
+  PRBF_CHECK_LAUNCH();
+}
+
 template <int DIM, int NV>
 void launch_sym(const GaussPlan& P, const PointsView& s, const double* gv, double* w, long long vs, unsigned* err,
                 const int* skip, cudaStream_t st) {
@@ -1489,9 +1520,7 @@ void launch_sym(const GaussPlan& P, const PointsView& s, const double* gv, doubl
     launch_sym_k<DIM, NV, true>(P, s, gv, w, vs, err, skip, st);
   else
     launch_sym_k<DIM, NV, false>(P, s, gv, w, vs, err, skip, st);
-  const int gb = std::max(1, std::min(ceil_div(s.n, 256), 8 * 152));
-  k_sym_gather<<<gb, 256, 0, st>>>(s.n, NV, P.sym_K, P.sym_pstride, P.sym_part.get(), w, vs, skip);
-  PRBF_CHECK_LAUNCH();
+  launch_sym_gather(P, s.n, NV, w, vs, skip, st);
 }
 
 template <int DIM>
@@ -1575,22 +1604,40 @@ void launch_nv(const GaussPlan& P, const PointsView& t, const PointsView& s, con
 // The FP32 form's masks hold 2 nb_trunc + 1 bits per axis and the cell y in 16 bits.
 static bool f32_grid_ok(const Grid& g) { return 2 * g.nb_trunc + 1 <= kMaskBits && g.ny < 65536; }
 
-static void alloc_f32(GaussPlan& plan, int dim, int n, cudaStream_t s) {
+// Buffers of the sources' forms; the entries past the points (read by the aligned bulk
+// copies, never used) zeroed.
+static PointForms alloc_forms(GaussPlan& plan, int dim, int n, bool f32, bool fx, cudaStream_t s) {
   const long long n8 = (long long)n + 8;
-  plan.su.reserve(n8);
-  plan.sv.reserve(n8);
-  plan.sw.reserve(dim == 3 ? n8 : 1);
-  plan.smask.reserve(n8);
-  plan.g32_stride = ((long long)n + 8 + 31) / 32 * 32;
-  plan.g32.reserve(4 * plan.g32_stride);
-  PRBF_CUDA(cudaMemsetAsync(plan.g32.get(), 0, sizeof(float) * 4 * plan.g32_stride, s));
-  for (auto* b : {&plan.su, &plan.sv}) PRBF_CUDA(cudaMemsetAsync(b->get(), 0, sizeof(float) * n8, s));
-  if (dim == 3) PRBF_CUDA(cudaMemsetAsync(plan.sw.get(), 0, sizeof(float) * n8, s));
-  PRBF_CUDA(cudaMemsetAsync(plan.smask.get(), 0, sizeof(unsigned long long) * n8, s));
+  PointForms o;
+  auto tail = [&](void* p, size_t elem) { PRBF_CUDA(cudaMemsetAsync((char*)p + elem * n, 0, elem * 8, s)); };
+  if (f32 || fx) {
+    o.mask = plan.smask.reserve(n8);
+    tail(o.mask, 8);
+  }
+  if (f32) {
+    o.u = plan.su.reserve(n8);
+    o.v = plan.sv.reserve(n8);
+    o.w = plan.sw.reserve(dim == 3 ? n8 : 1);
+    tail(o.u, 4);
+    tail(o.v, 4);
+    if (dim == 3) tail(o.w, 4);
+    plan.g32_stride = (n8 + 31) / 32 * 32;
+    plan.g32.reserve(4 * plan.g32_stride);
+    PRBF_CUDA(cudaMemset2DAsync(plan.g32.get() + n, sizeof(float) * plan.g32_stride, 0,
+                                sizeof(float) * (plan.g32_stride - n), 4, s));
+  }
+  if (fx) {
+    uint2** q[3] = {&o.fx, &o.fy, &o.fz};
+    for (int d = 0; d < dim; d++) {
+      *q[d] = plan.fxs[d].reserve(n8);
+      tail(*q[d], 8);
+    }
+  }
+  return o;
 }
 
 void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& src, unsigned* err,
-                    Workspace& ws, cudaStream_t s, bool forms) {
+                    Workspace& ws, cudaStream_t s, int forms) {
   (void)err;
   const Grid& g = plan.g;
   int* cnt = (int*)ws.get(20, sizeof(int) * ((size_t)g.ncell + 1));
@@ -1623,26 +1670,43 @@ void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& sr
   plan.max_trunc = h.maxc;
   plan.max_tile = kTileT;
   upload_table(s);
-  // FP32 form's source data
-  plan.f32_ready = false;
+  plan.f32_ready = plan.fx_ready = false;
   plan.sym_ready = false;
   plan.sym_nitems = 0;
   plan.sym_ncs = 0;
   if (!forms) return;
+  const bool self = tgt.x == src.x && tgt.n == src.n;
   if (f32_grid_ok(g) && src.n > 0) {
-    alloc_f32(plan, g.dim, src.n, s);
-    const SumConsts k32 = sum_consts(g.sigma, true, 0);
-    k_src_f32<<<ceil_div(g.ncell, 128), 128, 0, s>>>(g, src.cell_start, src.x, src.y, src.z, k32.scale,
-                                                     plan.su.get(), plan.sv.get(), plan.sw.get(), plan.smask.get());
+    const bool f32 = forms & FORM_F32, fx = (forms & FORM_F64) && fx_grid_ok(g);
+    const PointForms o = alloc_forms(plan, g.dim, src.n, f32, fx, s);
+    k_point_forms<<<ceil_div(g.ncell, 8), 256, 0, s>>>(g, nullptr, nullptr, g.ncell, src.cell_start, src.x, src.y,
+                                                       src.z, o);
     PRBF_CHECK_LAUNCH();
-    plan.f32_ready = true;
+    if (fx) {
+      gauss_fx_upload_tables(s);
+      plan.fx_self = self;
+      plan.fx_ncs = g.ncell + 1;
+      if (!self) {
+        PointForms ot;
+        uint2** q[3] = {&ot.fx, &ot.fy, &ot.fz};
+        for (int d = 0; d < g.dim; d++) *q[d] = plan.fxt[d].reserve(std::max(tgt.n, 1));
+        k_point_forms<<<ceil_div(g.ncell, 8), 256, 0, s>>>(g, nullptr, nullptr, g.ncell, tgt.cell_start, tgt.x, tgt.y,
+                                                           tgt.z, ot);
+        PRBF_CHECK_LAUNCH();
+      }
+    }
+    plan.f32_ready = f32;
+    plan.fx_ready = fx;
   }
+  // (the fixed-point form's symmetric sum is 2D, one vector: with more vectors, or 3D's wider
+  // windows, its one-sided sum is bound by the same multiply-adds and writes no slots)
+  if (!(forms & FORM_F64) || (plan.fx_ready && (g.dim == 3 || plan.sym_nv > 1))) return;
   // symmetric FP64 matvec: the same point set on both sides, every cell within one item
   // (<= kTileT points), 2 nb + 1 mask bits per axis, at most kSymMaxK partial slots per
   // point and vector (each product writes and gathers them: the 7 x 7 x 7 window of a 3D
   // cutoff of 2.8 cells has 171, whose traffic costs more than the halved exponentials
   // save), and the slots within 1/8 of the free device memory
-  if (tgt.x == src.x && tgt.n == src.n && src.n > 0 && 2 * g.nb_trunc + 1 <= kMaskBits && (g.dim == 2 || g.dim == 3)) {
+  if (self && src.n > 0 && 2 * g.nb_trunc + 1 <= kMaskBits) {
     int* dmax = (int*)ws.get(25, sizeof(int));
     PRBF_CUDA(cudaMemsetAsync(dmax, 0, sizeof(int), s));
     k_max_cell<<<ceil_div(g.ncell, 256), 256, 0, s>>>(g.ncell, src.cell_start, dmax);
@@ -1656,18 +1720,22 @@ void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& sr
     size_t free_b = 0, total_b = 0;
     PRBF_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const int nvs = std::max(1, std::min(4, plan.sym_nv));
-    const double bytes = (double)K * nvs * pstride * sizeof(double) + (double)(src.n + 8) * 8;
+    const int sets = plan.fx_ready && hmax > kFxSymTile ? 2 : 1;
+    const double bytes = (double)K * sets * nvs * pstride * sizeof(double) + (double)(src.n + 8) * 8;
     if (hmax <= kTileT && K >= 1 && K <= kSymMaxK && bytes <= 0.125 * (double)free_b) {
       plan.sym_K = K;
+      plan.sym_sets = sets;
       plan.sym_nv = nvs;
       plan.sym_pstride = pstride;
-      plan.sym_part.reserve((size_t)K * nvs * pstride);
-      PRBF_CUDA(cudaMemsetAsync(plan.sym_part.get(), 0, sizeof(double) * (size_t)K * nvs * pstride, s));
-      plan.sym_cy.reserve((size_t)src.n + 8);
-      PRBF_CUDA(cudaMemsetAsync(plan.sym_cy.get(), 0, sizeof(unsigned long long) * ((size_t)src.n + 8), s));
-      k_cell_y<<<std::max(1, std::min(ceil_div(g.ncell, 256), 8 * 152)), 256, 0, s>>>(g, src.cell_start,
-                                                                                   plan.sym_cy.get());
-      PRBF_CHECK_LAUNCH();
+      plan.sym_part.reserve((size_t)K * sets * nvs * pstride);
+      PRBF_CUDA(cudaMemsetAsync(plan.sym_part.get(), 0, sizeof(double) * (size_t)K * sets * nvs * pstride, s));
+      if (!plan.fx_ready) {
+        plan.sym_cy.reserve((size_t)src.n + 8);
+        PRBF_CUDA(cudaMemsetAsync(plan.sym_cy.get(), 0, sizeof(unsigned long long) * ((size_t)src.n + 8), s));
+        k_cell_y<<<std::max(1, std::min(ceil_div(g.ncell, 256), 8 * 152)), 256, 0, s>>>(g, src.cell_start,
+                                                                                     plan.sym_cy.get());
+        PRBF_CHECK_LAUNCH();
+      }
       plan.sym_ready = true;
     }
   }
@@ -1677,7 +1745,7 @@ bool gauss_plan_sym_batch(GaussPlan& plan, const std::vector<Grid>& grids, const
                           const std::vector<int>& hcs, cudaStream_t s) {
   plan.sym_ready = false;
   plan.sym_nitems = 0;
-  if (grids.empty() || src.n <= 0) return false;
+  if (grids.empty() || src.n <= 0 || (plan.fx_ready && grids[0].dim == 3)) return false;
   const int nb = grids[0].nb_trunc, dim = grids[0].dim;
   for (const Grid& g : grids)
     if (g.nb_trunc != nb || 2 * nb + 1 > kMaskBits) return false;
@@ -1687,9 +1755,11 @@ bool gauss_plan_sym_batch(GaussPlan& plan, const std::vector<Grid>& grids, const
   // one item per non-empty cell, each cell within one item; largest first
   std::vector<int2> its;
   const int ncell = (int)hcs.size() - 1;
+  int sets = 1;
   for (int c = 0; c < ncell; c++) {
     const int m = hcs[c + 1] - hcs[c];
     if (m > kTileT) return false;
+    if (plan.fx_ready && m > kFxSymTile) sets = 2;
     if (m > 0) its.push_back(make_int2(c, hcs[c]));
   }
   std::stable_sort(its.begin(), its.end(),
@@ -1697,19 +1767,22 @@ bool gauss_plan_sym_batch(GaussPlan& plan, const std::vector<Grid>& grids, const
   const long long pstride = ((long long)src.n + 8 + 31) / 32 * 32;
   size_t free_b = 0, total_b = 0;
   PRBF_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  if ((double)K * pstride * sizeof(double) + (double)(src.n + 8) * 8 > 0.125 * (double)free_b) return false;
+  if ((double)K * sets * pstride * sizeof(double) + (double)(src.n + 8) * 8 > 0.125 * (double)free_b) return false;
   plan.sym_K = K;
+  plan.sym_sets = sets;
   plan.sym_nv = 1;
   plan.sym_ncs = (int)hcs.size();
   plan.sym_pstride = pstride;
-  plan.sym_part.reserve((size_t)K * pstride);
-  PRBF_CUDA(cudaMemsetAsync(plan.sym_part.get(), 0, sizeof(double) * (size_t)K * pstride, s));
-  plan.sym_cy.reserve((size_t)src.n + 8);
-  PRBF_CUDA(cudaMemsetAsync(plan.sym_cy.get(), 0, sizeof(unsigned long long) * ((size_t)src.n + 8), s));
-  for (const Grid& g : grids)
-    k_cell_y<<<std::max(1, std::min(ceil_div(g.ncell, 256), 8 * 152)), 256, 0, s>>>(g, src.cell_start + g.cbase,
-                                                                                  plan.sym_cy.get());
-  PRBF_CHECK_LAUNCH();
+  plan.sym_part.reserve((size_t)K * sets * pstride);
+  PRBF_CUDA(cudaMemsetAsync(plan.sym_part.get(), 0, sizeof(double) * (size_t)K * sets * pstride, s));
+  if (!plan.fx_ready) {
+    plan.sym_cy.reserve((size_t)src.n + 8);
+    PRBF_CUDA(cudaMemsetAsync(plan.sym_cy.get(), 0, sizeof(unsigned long long) * ((size_t)src.n + 8), s));
+    for (const Grid& g : grids)
+      k_cell_y<<<std::max(1, std::min(ceil_div(g.ncell, 256), 8 * 152)), 256, 0, s>>>(g, src.cell_start + g.cbase,
+                                                                                    plan.sym_cy.get());
+    PRBF_CHECK_LAUNCH();
+  }
   plan.sym_items.reserve(std::max<size_t>(its.size(), 1));
   PRBF_CUDA(cudaMemcpyAsync(plan.sym_items.get(), its.data(), sizeof(int2) * its.size(), cudaMemcpyHostToDevice, s));
   PRBF_CUDA(cudaStreamSynchronize(s));
@@ -1718,21 +1791,27 @@ bool gauss_plan_sym_batch(GaussPlan& plan, const std::vector<Grid>& grids, const
   return true;
 }
 
-void gauss_plan_f32_batch(GaussPlan& plan, const std::vector<Grid>& grids, const PointsView& src, cudaStream_t s) {
-  plan.f32_ready = false;
+void gauss_plan_forms_batch(GaussPlan& plan, const std::vector<Grid>& grids, const PointsView& src, int forms,
+                            cudaStream_t s) {
+  plan.f32_ready = plan.fx_ready = false;
   if (src.n <= 0) return;
-  for (const Grid& g : grids)
-    if (!f32_grid_ok(g)) return;
-  alloc_f32(plan, grids[0].dim, src.n, s);
+  bool fx = forms & FORM_F64;
+  int ncell = 0;
   for (const Grid& g : grids) {
-    // the problem's cells are cell_start[cbase .. cbase + ncell]; its points keep their
-    // global positions
-    const SumConsts k32 = sum_consts(g.sigma, true, 0);
-    k_src_f32<<<ceil_div(g.ncell, 128), 128, 0, s>>>(g, src.cell_start + g.cbase, src.x, src.y, src.z, k32.scale,
-                                                     plan.su.get(), plan.sv.get(), plan.sw.get(), plan.smask.get());
-    PRBF_CHECK_LAUNCH();
+    if (!f32_grid_ok(g)) return;
+    fx = fx && fx_grid_ok(g);
+    ncell += g.ncell;
   }
-  plan.f32_ready = true;
+  const bool f32 = forms & FORM_F32;
+  const PointForms o = alloc_forms(plan, grids[0].dim, src.n, f32, fx, s);
+  k_point_forms<<<ceil_div(ncell, 8), 256, 0, s>>>(plan.g, plan.grids.get(), plan.cprob.get(), ncell, src.cell_start,
+                                                   src.x, src.y, src.z, o);
+  PRBF_CHECK_LAUNCH();
+  if (fx) gauss_fx_upload_tables(s);
+  plan.fx_self = true;
+  plan.fx_ncs = ncell + 1;
+  plan.f32_ready = f32;
+  plan.fx_ready = fx;
 }
 
 void gauss_sum_dev(const GaussPlan& P, const PointsView& t, const PointsView& s, const double* gv,
@@ -1742,10 +1821,18 @@ void gauss_sum_dev(const GaussPlan& P, const PointsView& t, const PointsView& s,
   if (nv > 1 && (vstride % 2 || vstride < t.n || vstride < s.n))
     throw Error(PRBF_ERR_ARG, "vector stride must be even and cover the points");
   if (!fp32 && P.sym_ready && std::min(nv, 4) <= P.sym_nv && t.x == s.x && t.n == s.n) {
-    if (P.g.dim == 2)
+    if (P.fx_ready) {
+      gauss_fx_sym(P, s, gv, w, err, skip, st);
+      launch_sym_gather(P, s.n, 1, w, 0, skip, st);
+    } else if (P.g.dim == 2) {
       launch_sym_nv<2>(P, s, gv, w, nv, vstride, err, skip, st);
-    else
+    } else {
       launch_sym_nv<3>(P, s, gv, w, nv, vstride, err, skip, st);
+    }
+    return;
+  }
+  if (!fp32 && P.fx_ready) {
+    gauss_fx_sum(P, t, s, gv, w, err, skip, nv, vstride, st);
     return;
   }
   if (P.g.dim == 2) {
