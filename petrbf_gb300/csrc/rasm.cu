@@ -352,58 +352,82 @@ __device__ void acc_to_smem(T* C, const T acc[4][4], TileMap mp = tile_map(false
     for (int q = 0; q < 4; q++) C[(ty * 4 + p) * S + tx * 4 + q] = acc[p][q];
 }
 
-// Ordered form of the diagonal-tile Cholesky (plain FP64 factor form): the h x h leading
-// part of C (lower) becomes L_kk in place, rd[j] = 1 / L_kk[j][j]. Column j: s = sqrt(c_jj),
-// r = 1/s, l_ij = c_ij * r, then c_il = fma(-l_ij, l_lj, c_il) for j < l <= i. Every entry
-// thus receives its updates in ascending column order, each one rounding, exactly as the
-// unblocked right-looking Cholesky with those operations computes it. Returns false if a
-// pivot is not positive (it is then taken as 1 and the block retried with a shift).
-// Entries outside h x h are set to the identity.
+// Ordered form of the diagonal-tile Cholesky (plain FP64 factor form): the h x h tile in the
+// threads' 4 x 4 blocks (tile_map(true)) becomes L_kk in C (lower; the identity outside h x h,
+// zeros above), rd[j] = 1 / L_kk[j][j]. Column j: s = sqrt(c_jj), r = 1/s, l_ij = c_ij * r, then
+// c_il = fma(-l_ij, l_lj, c_il) for j < l <= i. Every entry thus receives its updates in
+// ascending column order, each one rounding, exactly as the unblocked right-looking Cholesky
+// with those operations computes it. Returns false if a pivot is not positive (it is then taken
+// as 1 and the block retried with a shift).
+// Bound by the FP64 pipe, which takes 64 clocks of a sub-partition for a warp instruction
+// however few of its lanes are on: so one thread takes a column's root and reciprocal (about 25
+// such instructions; every thread computing them made them 200, two thirds of the tile), two
+// warps scale the column, and the tile stays in registers of the 136 threads that own lower
+// blocks, whose warps drop out as the column passes their rows.
 template <class T>
-__device__ bool potrf_rd(T* C, T* rd, int h) {
+__device__ bool potrf_rd(T acc[4][4], TileMap mp, T* C, T* rd, int h) {
   constexpr int S = SP<T>::S;
+  __shared__ T s_raw[TB], s_col[TB];
+  __shared__ T s_sq, s_rc;
   __shared__ int s_bad;
   if (threadIdx.x == 0) s_bad = 0;
-  __syncthreads();
   for (int e = threadIdx.x; e < TB * TB; e += NTH) {
-    int r = e / TB, c = e % TB;
-    if (r >= h || c >= h) C[r * S + c] = (r == c) ? T(1) : T(0);
-    if (c > r) C[r * S + c] = T(0);
-  }
-  __syncthreads();
-  const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-  for (int j = 0; j < h; j++) {
-    T d = C[j * S + j];
-    if (!(d > T(0))) {
-      if (threadIdx.x == 0) s_bad = 1;
-      d = T(1);
-    }
-    const T sq = sqrt(d);
-    const T rc = T(1) / sq;
-    __syncthreads();
-    for (int i = j + 1 + threadIdx.x; i < h; i += NTH) C[i * S + j] = C[i * S + j] * rc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      C[j * S + j] = sq;
-      rd[j] = rc;
-    }
-    T ci[4], cl[4];
-#pragma unroll
-    for (int p = 0; p < 4; p++) {
-      const int i = 4 * ty + p, l = 4 * tx + p;
-      ci[p] = (i > j && i < h) ? C[i * S + j] : T(0);
-      cl[p] = (l > j && l < h) ? C[l * S + j] : T(0);
-    }
-#pragma unroll
-    for (int p = 0; p < 4; p++)
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int i = 4 * ty + p, l = 4 * tx + q;
-        if (l > j && l <= i && i < h) C[i * S + l] = fma(-ci[p], cl[q], C[i * S + l]);
-      }
-    __syncthreads();
+    const int r = e / TB, c = e % TB;
+    if (r >= h || c >= h)
+      C[r * S + c] = (r == c) ? T(1) : T(0);
+    else if (c > r)
+      C[r * S + c] = T(0);
   }
   for (int j = h + threadIdx.x; j < TB; j += NTH) rd[j] = T(1);
+  __syncthreads();
+  const int i0 = 4 * mp.ty, l0 = 4 * mp.tx;
+  for (int j4 = 0; j4 < h; j4 += 4) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int j = j4 + q;
+      if (j >= h) break;
+      if (mp.on && l0 == j4) {  // the column's owners publish it unscaled, the pivot's its root
+#pragma unroll
+        for (int p = 0; p < 4; p++) s_raw[i0 + p] = acc[p][q];
+        if (i0 == j4) {
+          T d = acc[q][q];
+          if (!(d > T(0))) {
+            s_bad = 1;
+            d = T(1);
+          }
+          const T sq = sqrt(d);
+          s_sq = sq;
+          s_rc = T(1) / sq;
+        }
+      }
+      __syncthreads();
+      if (threadIdx.x < TB) {
+        const int i = threadIdx.x;
+        if (i == j) {
+          C[j * S + j] = s_sq;
+          rd[j] = s_rc;
+        } else if (i > j && i < h) {
+          const T v = s_raw[i] * s_rc;
+          s_col[i] = v;
+          C[i * S + j] = v;
+        }
+      }
+      __syncthreads();
+      if (mp.on && i0 + 3 > j) {
+        T ci[4], cl[4];
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+          ci[p] = (i0 + p > j && i0 + p < h) ? s_col[i0 + p] : T(0);
+          cl[p] = (l0 + p > j && l0 + p < h) ? s_col[l0 + p] : T(0);
+        }
+#pragma unroll
+        for (int p = 0; p < 4; p++)
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            if (l0 + u > j && l0 + u <= i0 + p && i0 + p < h) acc[p][u] = fma(-ci[p], cl[u], acc[p][u]);
+      }
+    }
+  }
   __syncthreads();
   return s_bad == 0;
 }
@@ -1093,15 +1117,24 @@ __global__ void __launch_bounds__(NTH) k_pack_factor(int nblk, const int* __rest
 }
 
 // ---- plain FP64 factor form: ordered block Cholesky -----------------------------------
-// One CTA per block: left-looking Cholesky of K over uniform 64 x 64 tiles. A tile starts
-// from K, receives the trailing updates of the earlier tile columns in ascending column
-// order (tile_update accumulates into the tile itself), and is then finished by potrf_rd
-// (diagonal tile) or trsm_rows (tiles below it). Every entry of L thus sees exactly the
-// operation sequence of the unblocked right-looking Cholesky written with fma, sqrt and
-// reciprocal pivots -- a CPU restatement of that loop reproduces the factor bit for bit.
+// A cluster of CTAs per block (one CTA where the blocks fill the GPU by themselves, see
+// chol_cluster): left-looking Cholesky of K over 64-column tiles. A tile starts from K, receives
+// the trailing updates of the earlier columns in ascending order (tile_update accumulates into
+// the tile itself), and is then finished by potrf_rd (the diagonal tile, by the cluster's first
+// CTA) or trsm_rows (tiles below it, whose rows the CTAs share out evenly, column by column).
+// Every entry of L thus sees exactly the operation sequence of the unblocked right-looking
+// Cholesky written with fma, sqrt and reciprocal pivots, whatever the tiles and CTAs -- a CPU
+// restatement of that loop reproduces the factor bit for bit.
 // The factor is then packed as the apply reads it: row i holds L_A[i][0..i-1] and
 // 1 / L_A[i][i], L_A = L_K sqrt(1 / (2 pi sigma^2)) the factor of A = K / (2 pi sigma^2).
-__global__ void __launch_bounds__(NTH, 2) k_chol_fp64(int nblk, const int* __restrict__ blk_cell,
+// Bound by the FP64 pipe. Measured, one CTA per block with every thread taking the pivots'
+// roots -> this form: 100 blocks of 900 (10^4 points in 2D, 3 CTAs a block) 39.8 -> 25.7 ms;
+// 343 blocks of up to 729 (26^3 in 3D, 3 CTAs) 35.7 -> 25.6 ms; 1576 blocks of 900 (one CTA)
+// 364.6 -> 345.5 ms; 34000 blocks of 144 to 225 (a batch in 2D, one CTA) 165.6 -> 108.5 ms.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+__global__ void __launch_bounds__(NTH, 2) k_chol_fp64(int nblk, int ncl, const int* __restrict__ blk_cell,
                                                    const long long* __restrict__ boff,
                                                    const long long* __restrict__ koff, double* __restrict__ K,
                                                    double out_scale_all, const double* __restrict__ cell_sig,
@@ -1109,7 +1142,7 @@ __global__ void __launch_bounds__(NTH, 2) k_chol_fp64(int nblk, const int* __res
                                                    const unsigned char* __restrict__ only,
                                                    const long long* __restrict__ loff, double* __restrict__ Lpack) {
   using T = double;
-  const int b = blockIdx.x;
+  const int b = blockIdx.x / ncl, rank = blockIdx.x % ncl;  // (clusters are consecutive CTAs)
   if (b >= nblk || (only && !only[b])) return;
   double out_scale = out_scale_all;  // sqrt(1 / (2 pi sigma^2)), per cell for a batch
   if (cell_sig) {
@@ -1127,53 +1160,103 @@ __global__ void __launch_bounds__(NTH, 2) k_chol_fp64(int nblk, const int* __res
   t.M = t.C + TB * S;
   const int c = blk_cell[b];
   const int nb = (int)(boff[c + 1] - boff[c]);
-  const int ntile = (nb + TB - 1) / TB;
   T* A = K + koff[b];
   bool ok = true;
-  for (int k = 0; k < ntile; k++) {
-    const int rk = k * TB, hk = min(TB, nb - rk);
-    for (int i = k; i < ntile; i++) {
-      const int ri = i * TB, hi = min(TB, nb - ri);
-      const TileMap mp = tile_map(i == k);  // a diagonal tile: its lower blocks only
-      T acc[4][4];
-      load_acc<T>(A, nb, ri, rk, hi, hk, acc, true, mp);
-      for (int p = 0; p < k; p++) {
-        const int rp = p * TB, hp = min(TB, nb - rp);
-        tile_update<T>(t, acc, A, nb, ri, rp, hi, false, A, nb, rk, rp, hk, false, hp, mp);
+  for (int rk = 0; rk < nb; rk += TB) {
+    const int hk = min(TB, nb - rk), below = nb - rk - hk;
+    // this CTA's rows below the diagonal tile: even shares in steps of 8 rows, the first CTA's
+    // less by the 48 that the diagonal tile counts for
+    int ra = 0, re = below;
+    if (ncl > 1) {
+      const int mine0 = min(below, max(0, (below + 48) / ncl - 48)) & ~7, rest = below - mine0;
+      ra = rank == 0 ? 0 : mine0 + ((int)((long long)rest * (rank - 1) / (ncl - 1)) & ~7);
+      re = rank == 0 ? mine0 : (rank == ncl - 1 ? below : mine0 + ((int)((long long)rest * rank / (ncl - 1)) & ~7));
+    }
+    T acc[4][4];
+    if (rank == 0) {
+      const TileMap mp = tile_map(true);  // its lower blocks only
+      load_acc<T>(A, nb, rk, rk, hk, hk, acc, true, mp);
+      tile_update<T>(t, acc, A, nb, rk, 0, hk, false, A, nb, rk, 0, hk, false, rk, mp);
+      __syncthreads();
+      ok = potrf_rd<T>(acc, mp, t.C, s_rd, hk) && ok;
+      // store L_kk and keep it in M for the panel solves of this tile column
+      for (int e = threadIdx.x; e < TB * TB; e += NTH) {
+        const int r = e / TB, cc = e % TB;
+        const T v = t.C[r * S + cc];
+        if (r < hk && cc <= r) A[(long long)(rk + r) * nb + rk + cc] = v;
+        t.M[r * S + cc] = v;
       }
       __syncthreads();
-      acc_to_smem<T>(t.C, acc, mp);  // potrf_rd zeroes the upper part it does not write
-      __syncthreads();
-      if (i == k) {
-        ok = potrf_rd<T>(t.C, s_rd, hk) && ok;
-        // store L_kk and keep it in M for the panel solves of this tile column
+    }
+    if (ncl > 1) cluster_arrive();  // the others wait for L_kk after their first tile's updates
+    bool have = rank == 0;
+    const int nt = (re - ra + TB - 1) / TB;
+    // tiles of a share are as even as they come, in steps of 8 rows
+    const int step = nt ? ((re - ra + nt - 1) / nt + 7) & ~7 : 0;
+    for (int i = 0; i < max(nt, 1); i++) {
+      const int r0 = min(re, ra + i * step), r1 = min(re, r0 + step);
+      const int ri = rk + hk + r0, hi = r1 - r0;
+      if (hi > 0) {
+        load_acc<T>(A, nb, ri, rk, hi, hk, acc, true);
+        tile_update<T>(t, acc, A, nb, ri, 0, hi, false, A, nb, rk, 0, hk, false, rk);
+      }
+      if (i == 0 && ncl > 1) cluster_wait();
+      if (hi <= 0) continue;
+      if (!have) {
+        have = true;
         for (int e = threadIdx.x; e < TB * TB; e += NTH) {
           const int r = e / TB, cc = e % TB;
-          const T v = t.C[r * S + cc];
-          if (r < hk && cc <= r) A[(long long)(rk + r) * nb + rk + cc] = v;
+          const bool in = r < hk && cc <= r;
+          const T v = in ? A[(long long)(rk + r) * nb + rk + cc] : (r == cc ? T(1) : T(0));
           t.M[r * S + cc] = v;
-        }
-      } else {
-        trsm_rows<T>(t.C, t.M, s_rd, hi, hk);
-        __syncthreads();
-        for (int e = threadIdx.x; e < TB * TB; e += NTH) {
-          const int r = e / TB, cc = e % TB;
-          if (r < hi && cc < hk) A[(long long)(ri + r) * nb + rk + cc] = t.C[r * S + cc];
+          if (r == cc) s_rd[r] = in ? T(1) / v : T(1);
         }
       }
       __syncthreads();
+      acc_to_smem<T>(t.C, acc);
+      __syncthreads();
+      trsm_rows<T>(t.C, t.M, s_rd, hi, hk);
+      __syncthreads();
+      for (int e = threadIdx.x; e < TB * TB; e += NTH) {
+        const int r = e / TB, cc = e % TB;
+        if (r < hi && cc < hk) A[(long long)(ri + r) * nb + rk + cc] = t.C[r * S + cc];
+      }
+      __syncthreads();
+    }
+    if (ncl > 1) {  // the column is complete
+      cluster_arrive();
+      cluster_wait();
     }
   }
   T* Lp = Lpack + loff[c];
   const T sc = (T)out_scale;
-  for (int i = 0; i < nb; i++) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = rank * (NTH / 32) + w; i < nb; i += ncl * (NTH / 32)) {
     const long long o = rowoff<T>(i);
-    for (int j = threadIdx.x; j <= i; j += NTH) {
+    for (int j = lane; j <= i; j += 32) {
       const T v = A[(long long)i * nb + j] * sc;
       Lp[o + j] = j == i ? T(1) / v : v;
     }
   }
-  if (threadIdx.x == 0) bad[b] = ok ? 0 : 1;
+  if (threadIdx.x == 0 && rank == 0) bad[b] = ok ? 0 : 1;
+}
+
+// CTAs per block of k_chol_fp64: the cluster size whose waves of the 2 x 152 resident CTAs take
+// least, a CTA's time counted as its share of the block (with 5 % for each further CTA: barriers,
+// uneven shares), twice that where two share an SM. One for blocks that fill many waves.
+int chol_cluster(int nblk) {
+  int best = 1;
+  double tbest = 1e300;
+  for (int n = 1; n <= 8; n++) {
+    const int per = 2 * 152 / n, full = nblk / per, rest = nblk - full * per;
+    const double w = (1.0 + 0.05 * (n - 1)) / n;
+    const double t = full * 2 * w + (rest == 0 ? 0.0 : rest * n <= 152 ? w : 2 * w);
+    if (t < 0.97 * tbest) {
+      tbest = t;
+      best = n;
+    }
+  }
+  return best;
 }
 
 // ---- apply: out[centre(c)] = S_c r[buffer(c) in block order] --------------------------
@@ -2047,9 +2130,21 @@ void rasm_factor(RasmPlan& R, const BlockGeom& G, const std::vector<int>& hcnt, 
                                               G.dim, inv2s2, G.cell_sigma, shift, (double*)Kw, only, nullptr, 0,
                                               kexp_of_sigma(G.sigma), exp_table_dev(s));
         PRBF_CHECK_LAUNCH();
-        k_chol_fp64<<<nb_batch, NTH, smem, s>>>(nb_batch, dbc, R.boff.get(), dk, (double*)Kw,
-                                                std::sqrt(1.0 / out_scale), G.cell_sigma, dbad, only, R.loff.get(),
-                                                R.L64.get());
+        const int ncl = chol_cluster(nb_batch);
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = ncl;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(nb_batch * ncl);
+        cfg.blockDim = dim3(NTH);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cfg.attrs = at;
+        cfg.numAttrs = ncl > 1 ? 1 : 0;
+        PRBF_CUDA(cudaLaunchKernelEx(&cfg, k_chol_fp64, nb_batch, ncl, (const int*)dbc, (const long long*)R.boff.get(),
+                                     (const long long*)dk, (double*)Kw, std::sqrt(1.0 / out_scale), G.cell_sigma, dbad,
+                                     only, (const long long*)R.loff.get(), R.L64.get()));
       }
       PRBF_CHECK_LAUNCH();
       hbad.resize(nb_batch);
