@@ -112,7 +112,8 @@ struct GaussPlan {
   // targets' where they are another point set
   bool fx_ready = false;
   bool fx_self = true;
-  int fx_ncs = 0;  // entries of the cell starts
+  bool pipe64 = false;  // FP64 sums by the FP64 pipe's kernels all the same (see solve.cu)
+  int fx_ncs = 0;       // entries of the cell starts
   DevBuf<uint2> fxs[3], fxt[3];
   // FP64 matvec with each exponential used for both rows (targets == sources, every cell
   // <= 128 points): K partial slots of pstride entries per weight vector, for up to sym_nv

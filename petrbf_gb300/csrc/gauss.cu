@@ -1831,7 +1831,7 @@ void gauss_sum_dev(const GaussPlan& P, const PointsView& t, const PointsView& s,
     }
     return;
   }
-  if (!fp32 && P.fx_ready) {
+  if (!fp32 && P.fx_ready && !P.pipe64) {
     gauss_fx_sum(P, t, s, gv, w, err, skip, nv, vstride, st);
     return;
   }

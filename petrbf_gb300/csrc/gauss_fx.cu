@@ -12,8 +12,7 @@
 // (bulk copies on an mbarrier, the next piece in flight while one is filtered), keeps those of
 // the cell's truncation set in order, and hands them on in two buffers of CfgX::KC sources. The
 // consumer warps own an even share of the pass's targets, at most CfgX::TG each, whose sums
-// stay in registers from the first buffer to the last; their lanes stride over a buffer's
-// sources. Nothing but the buffers' mbarriers joins the warps: with CTA barriers around the
+// stay in registers; their lanes stride over a buffer's sources. Nothing but the buffers' mbarriers joins the warps: with CTA barriers around the
 // filtering they spent a fifth of their time waiting there.
 // Measured against the FP64-pipe kernels of gauss.cu (one product, caller order): 2D, 4x10^6
 // points 44.7 -> 8.1 ms (79.8 -> 440 Gpairs/s); 3D, 96^3 points 180.7 -> 18.7 ms (39.5 -> 381).
@@ -106,7 +105,7 @@ __device__ __forceinline__ double fx_scatter_sum(const double (&a)[N], int lane,
 #pragma unroll
   for (int i = 0; i < P; i++) k[i] = i < N ? a[i] : 0.0;
   which = 0;
-  int bit = 1;
+  int bit = 16;
 #pragma unroll
   for (int h = P / 2; h >= 1; h /= 2) {
     const bool up = lane & bit;
@@ -116,10 +115,10 @@ __device__ __forceinline__ double fx_scatter_sum(const double (&a)[N], int lane,
       k[i] = mine + __shfl_xor_sync(F, other, bit);
     }
     which += up ? h : 0;
-    bit <<= 1;
+    bit >>= 1;
   }
-  for (; bit < 32; bit <<= 1) k[0] += __shfl_xor_sync(F, k[0], bit);
-  const int low = 32 - P;  // lanes that differ in these bits hold the same total
+  for (; bit > 0; bit >>= 1) k[0] += __shfl_xor_sync(F, k[0], bit);
+  const int low = 32 / P - 1;  // lanes that differ in these bits hold the same total
   if ((lane & low) != 0 || which >= N) which = -1;
   return k[0];
 }
@@ -177,6 +176,23 @@ __device__ __forceinline__ bool fx_consume(unsigned char* smem, FxShared& sh, co
     }
   }
   __syncwarp();
+  // after every buffer (one-sided form) the lanes' sums meet and join their target's running
+  // total: the partial sums stay short, as rounding grows with their length (a 3D target has
+  // some 10^4 sources)
+  double run[NV];
+  int which = -1;
+#pragma unroll
+  for (int v = 0; v < NV; v++) run[v] = 0.0;
+  auto join = [&]() {
+    if constexpr (N > 0) {
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        run[v] += fx_scatter_sum<N>(acc[v], lane, which);
+#pragma unroll
+        for (int k = 0; k < N; k++) acc[v][k] = 0.0;
+      }
+    }
+  };
   while (true) {
     if (!mbar_wait(&sh.full[b], ph)) return false;
     const int n = sh.n[b];
@@ -243,15 +259,13 @@ __device__ __forceinline__ bool fx_consume(unsigned char* smem, FxShared& sh, co
     if (lane == 0) mbar_arrive(&sh.empty[b]);
     ph ^= b;
     b ^= 1;
+    if (!SYM || last) join();
     if (last) break;
   }
-  if constexpr (N > 0)
+  if (N > 0 && which >= 0) {
 #pragma unroll
-    for (int v = 0; v < NV; v++) {
-      int k;
-      const double sum = fx_scatter_sum<N>(acc[v], lane, k);
-      if (k >= 0) a.w[v * a.vs + t + k] = sum * norm;
-    }
+    for (int v = 0; v < NV; v++) a.w[v * a.vs + t + which] = run[v] * norm;
+  }
   return true;
 }
 
