@@ -1287,164 +1287,204 @@ __global__ void __launch_bounds__(128) k_apply(int ncell, const long long* __res
   }
 }
 
-// ---- apply with the factor: out[centre(c)] = (L^-T L^-1 r_c)[centre] ----------------
-// Forward substitution over the whole block (32-row panels: warp 0 solves the diagonal
-// triangle from shared memory, all warps update the rows below with coalesced row
-// segments), then the back substitution with L22^T only, since the centre unknowns are
-// the last n_c: x2 = L22^-T y2. With full set (basic Schwarz) the back substitution runs
-// over the whole block and the whole solution goes to the block's slots of Y (slot =
-// position in the buffer list); k_asm_gather then sums each point's slots in block order,
-// so the result does not depend on the order the blocks ran in. NV right-hand sides
+// ---- FP64 apply with the factor: out[centre(c)] = (L^-T L^-1 r_c)[centre] ------------
+// Forward substitution over the whole block, then the back substitution with L22^T only, since
+// the centre unknowns are the last n_c: x2 = L22^-T y2. With full set (basic Schwarz) the back
+// substitution runs over the whole block and the whole solution goes to the block's slots of Y
+// (slot = position in the buffer list); k_asm_gather then sums each point's slots in block
+// order, so the result does not depend on the order the blocks ran in. NV right-hand sides
 // (vectors at stride vs, slots at stride ys) share every load of the factor.
-template <class T, int NV>
-__global__ void __launch_bounds__(256) k_apply_tri(int ncell, const long long* __restrict__ boff,
-                                                   const int* __restrict__ cs, const int* __restrict__ idx,
-                                                   const long long* __restrict__ loff, const T* __restrict__ Lpack,
-                                                   const double* __restrict__ r, double* __restrict__ out,
-                                                   long long vs, const int* __restrict__ skip, int full,
-                                                   double* __restrict__ Y, long long ys, SegSkip seg,
-                                                   const int* __restrict__ lu_of_cell) {
+//
+// One CTA per block, panels of 32 rows. Warp 0 updates the next panel's rows with the panel just
+// solved and solves its triangle while the other warps take the rows beyond, 32 at a time off a
+// shared counter: one barrier per panel, and the triangle's chain (a product, a broadcast and a
+// multiply-add for each of its rows) runs beside the updates instead of between them. The
+// operations on an entry and their order are those of the sequential loops
+//   forward: y_i = (y_i - sum_j fma L_ij y_j) / L_ii within the panel, then for the rows below
+//     y_i -= (s0 + s1) + (s2 + s3), s_q the fma sum of 8 of the panel's 32 columns;
+//   backward: the panel's triangle likewise, then y_k -= the panel's fma sum for the rows above
+// whatever warp does them, so a CPU restatement reproduces the result bit for bit.
+// Bound by the FP64 pipe (a warp instruction costs 64 clocks of a sub-partition however few of
+// its lanes are on): the sums of 32 rows by 32 columns are 36 instructions forward (four lanes a
+// row, their partial sums exchanged so that each lane ends with one row; reducing every row's by
+// itself took 44) and 33 backward, a triangle 32 (1 + NV).
+// Measured, an apply in one vector per launch and with the triangles between the updates -> this
+// form: 100 blocks of 900 (2D) 288 -> 138 us; 343 of up to 729 (3D), three vectors 2.1 -> 1.0 ms;
+// 1576 of 900 1.8 -> 1.6 ms; 34000 of 144 to 225 (a batch) 2.4 -> 2.0 ms.
+template <int NV>
+__global__ void __launch_bounds__(256, 2) k_apply_tri64(int ncell, const long long* __restrict__ boff,
+                                                     const int* __restrict__ cs, const int* __restrict__ idx,
+                                                     const long long* __restrict__ loff,
+                                                     const double* __restrict__ Lpack, const double* __restrict__ r,
+                                                     double* __restrict__ out, long long vs,
+                                                     const int* __restrict__ skip, int full, double* __restrict__ Y,
+                                                     long long ys, SegSkip seg, const int* __restrict__ lu_of_cell) {
   if (skip && *skip) return;
   if (seg.cell_done(blockIdx.x)) return;
   if (lu_of_cell && lu_of_cell[blockIdx.x] >= 0) return;  // factored by LU: k_apply_lu
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ T tri[32][33];
+  __shared__ double tri[32][33];
+  __shared__ int s_next[2];  // the next tile of 32 rows, for this panel and the following one
   const int c = blockIdx.x;
   const int nb = (int)(boff[c + 1] - boff[c]);
   if (nb == 0) return;
-  T* y = (T*)smem_raw;  // NV x nb
+  double* y = (double*)smem_raw;  // NV x nb
   const int nc = cs[c + 1] - cs[c], n1 = nb - nc;
   const int* id = idx + boff[c];
-  const T* L = Lpack + loff[c];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
+  const double* L = Lpack + loff[c];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  constexpr unsigned F = 0xffffffffu;
+  if (tid < 2) s_next[tid] = 0;
   for (int j = tid; j < nb; j += blockDim.x) {
     const int p = id[j < n1 ? nc + j : j - n1];
 #pragma unroll
-    for (int v = 0; v < NV; v++) y[v * nb + j] = (T)r[v * vs + p];
+    for (int v = 0; v < NV; v++) y[v * nb + j] = r[v * vs + p];
   }
+  // (warp 0) rows o .. o + np of the panel's triangle
+  auto load_tri = [&](int o, int np) {
+#pragma unroll 8
+    for (int i = 0; i < 32; i++) tri[i][lane] = (i < np && lane <= i) ? L[rowoff<double>(o + i) + o + lane] : 0.0;
+    __syncwarp();
+  };
+  // (warp 0) the triangle's solve, rows ascending (forward) or descending (backward: its
+  // transpose); the diagonal holds reciprocals. Lane v takes the pivot row's product of vector v.
+  auto solve_tri = [&](int o, int np, bool up) {
+    double x[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) x[v] = lane < np ? y[v * nb + o + lane] : 0.0;
+    for (int q = 0; q < np; q++) {
+      const int j = up ? np - 1 - q : q;
+      const double d = tri[j][j], l = up ? tri[j][lane] : tri[lane][j];
+      double pv = __shfl_sync(F, x[0], j);
+#pragma unroll
+      for (int v = 1; v < NV; v++) {
+        const double t = __shfl_sync(F, x[v], j);
+        pv = lane == v ? t : pv;
+      }
+      pv *= d;
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        const double xj = __shfl_sync(F, pv, v);
+        if (lane == j) x[v] = xj;
+        if (up ? lane < j : lane > j) x[v] = fma(-l, xj, x[v]);
+      }
+    }
+    if (lane < np)
+#pragma unroll
+      for (int v = 0; v < NV; v++) y[v * nb + o + lane] = x[v];
+    __syncwarp();
+  };
+  // rows i0 .. i0 + 31 (a warp), panel p0: rows below a panel only exist when it is full, so that
+  // a lane's 8 entries lie inside the row, 16-byte aligned
+  auto forward_tile = [&](int i0, int p0) {
+    const int sub = lane & 3, rw = lane >> 2;
+    double ysv[NV][8], acc[NV][4];
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+#pragma unroll
+      for (int q = 0; q < 8; q++) ysv[v][q] = y[v * nb + p0 + sub * 8 + q];
+#pragma unroll
+      for (int u = 0; u < 4; u++) acc[v][u] = 0.0;
+    }
+    double2 lv[2][4];
+    auto fetch = [&](int u, double2 (&d)[4]) {
+      const int i = i0 + 8 * u + rw;
+      const double2* Li = reinterpret_cast<const double2*>(L + rowoff<double>(i < nb ? i : nb - 1) + p0 + sub * 8);
+#pragma unroll
+      for (int q = 0; q < 4; q++) d[q] = Li[q];
+    };
+    fetch(0, lv[0]);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      if (u < 3) fetch(u + 1, lv[(u + 1) & 1]);
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+          acc[v][u] = fma(lv[u & 1][q].x, ysv[v][2 * q], acc[v][u]);
+          acc[v][u] = fma(lv[u & 1][q].y, ysv[v][2 * q + 1], acc[v][u]);
+        }
+    }
+    const bool h1 = lane & 1, h2 = lane & 2;
+    const int i = i0 + 8 * ((h1 ? 2 : 0) + (h2 ? 1 : 0)) + rw;
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      const double k0 = (h1 ? acc[v][2] : acc[v][0]) + __shfl_xor_sync(F, h1 ? acc[v][0] : acc[v][2], 1);
+      const double k1 = (h1 ? acc[v][3] : acc[v][1]) + __shfl_xor_sync(F, h1 ? acc[v][1] : acc[v][3], 1);
+      const double s = (h2 ? k1 : k0) + __shfl_xor_sync(F, h2 ? k0 : k1, 2);
+      if (i < nb) y[v * nb + i] -= s;
+    }
+  };
   __syncthreads();
   // forward: L y = r
-  for (int p0 = 0; p0 < nb; p0 += 32) {
-    const int np = min(32, nb - p0);
-    for (int e = tid; e < 32 * 32; e += blockDim.x) {
-      int i = e >> 5, j = e & 31;
-      tri[i][j] = (i < np && j <= i) ? L[rowoff<T>(p0 + i) + p0 + j] : T(0);
-    }
-    __syncthreads();
+  if (w == 0) {
+    load_tri(0, min(32, nb));
+    solve_tri(0, min(32, nb), false);
+  }
+  __syncthreads();
+  int turn = 0;
+  for (int p0 = 0; p0 + 32 < nb; p0 += 32, turn ^= 1) {
     if (w == 0) {
-      T ri[NV];
-#pragma unroll
-      for (int v = 0; v < NV; v++) ri[v] = lane < np ? y[v * nb + p0 + lane] : T(0);
-      for (int j = 0; j < np; j++) {
-        const T d = tri[j][j], l = tri[lane][j];
-#pragma unroll
-        for (int v = 0; v < NV; v++) {
-          if (lane == j) ri[v] = ri[v] * d;  // reciprocal diagonal
-          T yj = __shfl_sync(0xffffffffu, ri[v], j);
-          if (lane > j) ri[v] = fma(-l, yj, ri[v]);
-        }
-      }
-      if (lane < np)
-#pragma unroll
-        for (int v = 0; v < NV; v++) y[v * nb + p0 + lane] = ri[v];
+      if (lane == 0) s_next[turn ^ 1] = 0;
+      const int o = p0 + 32, np = min(32, nb - o);
+      load_tri(o, np);
+      forward_tile(o, p0);
+      __syncwarp();
+      solve_tri(o, np, false);
     }
-    __syncthreads();
-    // rows below the panel: y[i] -= L[i][p0 .. p0+np) . y[p0 ..]. Four lanes per row, each
-    // with 8 contiguous entries, so 8 rows per warp pass and 2 shuffle levels: on GB300's
-    // narrow FP64 pipe a full warp reduction per row would cost 5x the row's FMAs.
-    {
-      const int sub = lane & 3, rw = lane >> 2;
-      T ysv[NV][8];
-#pragma unroll
-      for (int v = 0; v < NV; v++)
-#pragma unroll
-        for (int q = 0; q < 8; q++) ysv[v][q] = (sub * 8 + q < np) ? y[v * nb + p0 + sub * 8 + q] : T(0);
-      for (int i0 = p0 + np + 8 * w; i0 < nb; i0 += 8 * nw) {
-        const long long i = i0 + rw;
-        T acc[NV];
-#pragma unroll
-        for (int v = 0; v < NV; v++) acc[v] = T(0);
-        if (i < nb) {
-          // rows below a panel only exist when the panel is full (np = 32): all 8 entries
-          // of the segment lie inside row i, 16-byte aligned
-          T lv[8];
-          const T* Li = L + rowoff<T>(i) + p0 + sub * 8;
-          if constexpr (sizeof(T) == 8) {
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-              const double2 t2 = reinterpret_cast<const double2*>(Li)[q];
-              lv[2 * q] = t2.x;
-              lv[2 * q + 1] = t2.y;
-            }
-          } else {
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-              const float4 t4 = reinterpret_cast<const float4*>(Li)[q];
-              lv[4 * q] = t4.x;
-              lv[4 * q + 1] = t4.y;
-              lv[4 * q + 2] = t4.z;
-              lv[4 * q + 3] = t4.w;
-            }
-          }
-#pragma unroll
-          for (int q = 0; q < 8; q++)
-#pragma unroll
-            for (int v = 0; v < NV; v++) acc[v] = fma(lv[q], ysv[v][q], acc[v]);
-        }
-#pragma unroll
-        for (int v = 0; v < NV; v++) {
-          acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], 1);
-          acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], 2);
-        }
-        if (sub == 0 && i < nb)
-#pragma unroll
-          for (int v = 0; v < NV; v++) y[v * nb + i] -= acc[v];
-      }
+    while (true) {
+      int t = 0;
+      if (lane == 0) t = atomicAdd(&s_next[turn], 1);
+      const int i0 = p0 + 64 + 32 * __shfl_sync(F, t, 0);
+      if (i0 >= nb) break;
+      forward_tile(i0, p0);
     }
     __syncthreads();
   }
   // backward on the trailing block (rows b0 ..): L22^T x2 = y2, panels from the bottom
   const int b0 = full ? 0 : n1, nback = nb - b0;
-  for (int pe = nback; pe > 0; pe -= 32) {
-    const int p0 = max(0, pe - 32), np = pe - p0;
-    // tri[i][j] = L22[p0 + i][p0 + j], j <= i
-    for (int e = tid; e < 32 * 32; e += blockDim.x) {
-      int i = e >> 5, j = e & 31;
-      long long row = b0 + p0 + i;
-      tri[i][j] = (i < np && j <= i) ? L[rowoff<T>(row) + b0 + p0 + j] : T(0);
+  auto backward_tile = [&](int k0, int kn, int p0) {  // columns k0 .. of the full panel at p0
+    const int k = k0 + lane;
+    double acc[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) acc[v] = 0.0;
+    const bool on = k < kn;
+#pragma unroll 16
+    for (int j = 0; j < 32; j++) {
+      const int row = b0 + p0 + j;
+      const double lv = L[rowoff<double>(row) + b0 + (on ? k : k0)];
+#pragma unroll
+      for (int v = 0; v < NV; v++) acc[v] = fma(lv, y[v * nb + row], acc[v]);
     }
-    __syncthreads();
-    if (w == 0) {  // x_i = (y_i - sum_{j > i} L22[j][i] x_j) / L22[i][i], i = np-1 .. 0
-      T xi[NV];
-#pragma unroll
-      for (int v = 0; v < NV; v++) xi[v] = lane < np ? y[v * nb + b0 + p0 + lane] : T(0);
-      for (int j = np - 1; j >= 0; j--) {
-        const T d = tri[j][j], l = tri[j][lane];
-#pragma unroll
-        for (int v = 0; v < NV; v++) {
-          if (lane == j) xi[v] = xi[v] * d;  // reciprocal diagonal
-          T xj = __shfl_sync(0xffffffffu, xi[v], j);
-          if (lane < j) xi[v] = fma(-l, xj, xi[v]);
-        }
-      }
-      if (lane < np)
-#pragma unroll
-        for (int v = 0; v < NV; v++) y[v * nb + b0 + p0 + lane] = xi[v];
-    }
-    __syncthreads();
-    // rows above the panel: y2[k] -= sum_{j in panel} L22[p0 + j][k] x_j, k < p0
-    for (int k = tid; k < p0; k += blockDim.x) {
-      T acc[NV];
-#pragma unroll
-      for (int v = 0; v < NV; v++) acc[v] = T(0);
-      for (int j = 0; j < np; j++) {
-        long long row = b0 + p0 + j;
-        const T lv = L[rowoff<T>(row) + b0 + k];
-#pragma unroll
-        for (int v = 0; v < NV; v++) acc[v] = fma(lv, y[v * nb + b0 + p0 + j], acc[v]);
-      }
+    if (on)
 #pragma unroll
       for (int v = 0; v < NV; v++) y[v * nb + b0 + k] -= acc[v];
+  };
+  if (w == 0) {
+    if (lane < 2) s_next[lane] = 0;
+    const int np = min(32, nback), o = b0 + nback - np;
+    if (np > 0) {
+      load_tri(o, np);
+      solve_tri(o, np, true);
+    }
+  }
+  __syncthreads();
+  turn = 0;
+  for (int p0 = nback - 32; p0 > 0; p0 -= 32, turn ^= 1) {
+    const int q0 = max(0, p0 - 32);  // the next panel
+    if (w == 0) {
+      if (lane == 0) s_next[turn ^ 1] = 0;
+      load_tri(b0 + q0, p0 - q0);
+      backward_tile(q0, p0, p0);
+      __syncwarp();
+      solve_tri(b0 + q0, p0 - q0, true);
+    }
+    while (true) {
+      int t = 0;
+      if (lane == 0) t = atomicAdd(&s_next[turn], 1);
+      const int k0 = 32 * __shfl_sync(F, t, 0);
+      if (k0 >= q0) break;
+      backward_tile(k0, q0, p0);
     }
     __syncthreads();
   }
@@ -1452,11 +1492,11 @@ __global__ void __launch_bounds__(256) k_apply_tri(int ncell, const long long* _
     double* Yc = Y + boff[c];
     for (int j = tid; j < nb; j += blockDim.x)
 #pragma unroll
-      for (int v = 0; v < NV; v++) Yc[v * ys + (j < n1 ? nc + j : j - n1)] = (double)y[v * nb + j];
+      for (int v = 0; v < NV; v++) Yc[v * ys + (j < n1 ? nc + j : j - n1)] = y[v * nb + j];
   } else {
     for (int i = tid; i < nc; i += blockDim.x)
 #pragma unroll
-      for (int v = 0; v < NV; v++) out[v * vs + cs[c] + i] = (double)y[v * nb + n1 + i];
+      for (int v = 0; v < NV; v++) out[v * vs + cs[c] + i] = y[v * nb + n1 + i];
   }
 }
 
@@ -1738,7 +1778,7 @@ __global__ void __launch_bounds__(kLuThreads) k_lu_fp64(int nlu, const int* __re
 // The LU blocks' share of an apply: y <- 2 pi sigma^2 K^-1 y in the entry-wise order of the
 // sequential solve (interchanges in order; forward, y_i receiving fma(-l_ik, y_k, .) for
 // ascending k; backward, descending k with the division by the pivot when y_k is final),
-// then the restricted (centre rows) or basic (all slots) output of k_apply_tri.
+// then the restricted (centre rows) or basic (all slots) output of k_apply_tri64.
 __global__ void __launch_bounds__(kLuThreads) k_apply_lu(int nlu, const int* __restrict__ lucell,
                                                          const long long* __restrict__ boff,
                                                          const int* __restrict__ cs, const int* __restrict__ idx,
@@ -1981,9 +2021,6 @@ void rasm_factor(RasmPlan& R, const BlockGeom& G, const std::vector<int>& hcnt, 
   const int ncell = G.ncell;
   R.fp32 = fp32;
   R.ncell = ncell;
-  // several right-hand sides per launch pay off in FP32 (the factor read is shared); the
-  // FP64 solves are bound by the FP64 pipe and lose occupancy with more vectors
-  if (!fp32) R.max_nv = 1;
   // host plan: offsets of S_c, the list of non-empty blocks (largest first, so the batches
   // of the factorisation keep similar sizes together and the long blocks start early)
   std::vector<long long> hso(ncell + 1);
@@ -2000,6 +2037,9 @@ void rasm_factor(RasmPlan& R, const BlockGeom& G, const std::vector<int>& hcnt, 
   }
   if (G.cell_sigma)
     std::stable_sort(blk.begin(), blk.end(), [&](int a, int b) { return hcnt[a] > hcnt[b]; });
+  // as many right-hand sides per launch as a block's vectors leave room for (FP64)
+  if (!fp32)
+    while (R.max_nv > 1 && (size_t)R.max_nv * R.max_nb * sizeof(double) > 100 * 1024) R.max_nv--;
   R.nblocks = (int)blk.size();
   R.soff.reserve(ncell + 1);
   PRBF_CUDA(cudaMemcpyAsync(R.soff.get(), hso.data(), sizeof(long long) * (ncell + 1), cudaMemcpyHostToDevice, s));
@@ -2171,6 +2211,17 @@ void rasm_factor(RasmPlan& R, const BlockGeom& G, const std::vector<int>& hcnt, 
 }
 
 namespace {
+// Threads of k_apply_tri64. Few blocks: eight warps each; many: four, so that the triangles of
+// some CTAs meet the updates of others; small blocks, whose panels keep no four warps busy, two
+// or, where they fill the SMs all the same, one. Applies timed with 32, 64, 96, 128, 256 threads
+// (ms): 100 blocks of 900 .. 0.47 0.25 0.19 0.16 0.14; 343 of up to 729, three vectors 3.3 1.8 1.4
+// 1.2 1.0; 4225 of 900 5.0 3.8 3.9 3.9 5.0; 1728 of up to 729, three vectors 5.4 4.3 4.0 3.9 4.4;
+// 34000 of 144 to 225 2.0 2.2 2.7 3.1 5.7.
+int tri64_threads(const RasmPlan& R) {
+  if (R.max_nb <= 256) return R.nblocks >= 17 * 152 ? 32 : R.nblocks >= 4 * 152 ? 64 : 128;
+  return R.nblocks >= 3 * 152 ? 128 : 256;
+}
+
 int trw_ldy(const RasmPlan& R) { return (std::max(R.max_nb, 1) + 3) & ~3; }
 
 template <class T>
@@ -2200,26 +2251,11 @@ void apply_tri_nv(const RasmPlan& R, const T* Lp, const int* cs, const double* r
         break;
     }
   } else {
-    const size_t sm = (size_t)nv * R.max_nb * sizeof(T);
+    const size_t sm = (size_t)nv * R.max_nb * sizeof(double);
     const int* luc = R.nlu ? R.lu_of_cell.get() : nullptr;
-    switch (nv) {
-      case 1:
-        k_apply_tri<T, 1><<<R.ncell, 256, sm, s>>>(R.ncell, R.boff.get(), cs, R.idx.get(), R.loff.get(), Lp, r, out,
-                                                   vs, skip, full, R.Y.get(), R.nslot, R.seg, luc);
-        break;
-      case 2:
-        k_apply_tri<T, 2><<<R.ncell, 256, sm, s>>>(R.ncell, R.boff.get(), cs, R.idx.get(), R.loff.get(), Lp, r, out,
-                                                   vs, skip, full, R.Y.get(), R.nslot, R.seg, luc);
-        break;
-      case 3:
-        k_apply_tri<T, 3><<<R.ncell, 256, sm, s>>>(R.ncell, R.boff.get(), cs, R.idx.get(), R.loff.get(), Lp, r, out,
-                                                   vs, skip, full, R.Y.get(), R.nslot, R.seg, luc);
-        break;
-      default:
-        k_apply_tri<T, 4><<<R.ncell, 256, sm, s>>>(R.ncell, R.boff.get(), cs, R.idx.get(), R.loff.get(), Lp, r, out,
-                                                   vs, skip, full, R.Y.get(), R.nslot, R.seg, luc);
-        break;
-    }
+    const auto k = nv == 1 ? k_apply_tri64<1> : nv == 2 ? k_apply_tri64<2> : nv == 3 ? k_apply_tri64<3> : k_apply_tri64<4>;
+    k<<<R.ncell, tri64_threads(R), sm, s>>>(R.ncell, R.boff.get(), cs, R.idx.get(), R.loff.get(), Lp, r, out, vs, skip,
+                                            full, R.Y.get(), R.nslot, R.seg, luc);
   }
   PRBF_CHECK_LAUNCH();
 }
@@ -2235,9 +2271,9 @@ void set_tri_smem(const RasmPlan& R) {
                   : nv == 2 ? (const void*)k_apply_trw<2> : nv == 3 ? (const void*)k_apply_trw<3> : (const void*)k_apply_trw<4>;
     } else {
       sm = (size_t)nv * std::max(R.max_nb, 1) * sizeof(T) + sizeof(T) * 32 * 33;
-      f = nv == 1 ? (const void*)k_apply_tri<T, 1>
-                  : nv == 2 ? (const void*)k_apply_tri<T, 2>
-                            : nv == 3 ? (const void*)k_apply_tri<T, 3> : (const void*)k_apply_tri<T, 4>;
+      f = nv == 1 ? (const void*)k_apply_tri64<1>
+                  : nv == 2 ? (const void*)k_apply_tri64<2>
+                            : nv == 3 ? (const void*)k_apply_tri64<3> : (const void*)k_apply_tri64<4>;
     }
     if (sm > 220 * 1024) throw Error(PRBF_ERR_CAPACITY, "subdomain larger than the apply kernel's shared memory");
     PRBF_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,

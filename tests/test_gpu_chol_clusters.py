@@ -1,6 +1,6 @@
 """The FP64 block Cholesky with one to eight CTAs per block: the number of blocks picks the
 cluster, so point sets of few and many cells with blocks of ragged sizes (tiles' edges at 64,
-row shares of 8), each compared bit for bit with the restated block arithmetic through the
+row shares of 8; the apply's CTAs of one to eight warps), each compared bit for bit with the restated block arithmetic through the
 Schwarz apply."""
 import numpy as np
 import pytest
@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("pc", ["rasm", "asm"])
 @pytest.mark.parametrize("cells,most", [(1, 1), (1, 63), (1, 64), (1, 65), (1, 129), (2, 200), (13, 150), (30, 260),
-                                        (60, 90), (100, 140), (152, 60), (220, 70), (310, 66)])
+                                        (60, 90), (100, 140), (152, 60), (220, 70), (310, 66),
+                                        (700, 20), (2700, 9)])
 def test_applies_equal_the_restatement(cells, most, pc):
     rng = np.random.default_rng(cells * 1000 + most)
     prm = (0.0175, 22, 30, 24)  # lattice steps of 1.3 sigma and more: no shifted blocks
