@@ -1,10 +1,14 @@
 // gemm_tc.cu -- the learned-guess network's GEMMs on the tensor cores (sm_103a):
 //
 //   C[M][N] = A[M][K] B[N][K]^T  (+ bias[n], ReLU)   A, B BF16 row-major (K contiguous),
-//                                                    FP32 accumulation, FP32 and/or BF16 out
+//                                                    FP32 accumulation, FP32 and/or BF16 out,
+//                                                    the BF16 also transposed
 //
-// One CTA computes a 128-row tile with the whole N (<= 256) as one tcgen05.mma.kind::f16
-// accumulator in TMEM. The K dimension runs in chunks of 64 BF16 (128 bytes): warp 0
+// One CTA computes a 128-row tile of BN columns as one tcgen05.mma.kind::f16 accumulator in
+// TMEM, several products of one launch along the grid's z. Many row tiles: the whole N (<= 256)
+// per CTA, each row of A read once; few (a training batch of 512 rows has four): 64 columns, so
+// that four times the CTAs share the epilogue, which is what such a product takes (512 rows by
+// 256 columns, K = 256: 18.8 us as four CTAs, 10.1 us as sixteen). The K dimension runs in chunks of 64 BF16 (128 bytes): warp 0
 // stages each chunk of A (128 x 64) and B (BN x 64) with two tiled TMA copies
 // (cp.async.bulk.tensor, 128-byte swizzle, zero fill past the matrix edges) into a ring of
 // shared-memory stages that complete on mbarriers; warp 1 issues the four K = 16 MMAs of a
@@ -15,6 +19,8 @@
 #include <cuda.h>  // CUtensorMap and its enums (the encoder comes from the runtime's entry point)
 #include <cuda_bf16.h>
 
+#include <algorithm>
+#include <atomic>
 #include <mutex>
 
 #include "device.h"
@@ -25,7 +31,8 @@ namespace {
 
 constexpr int GM = 128;     // rows per CTA (TMEM lanes)
 constexpr int GKC = 64;     // K per stage: 64 BF16 = 128 bytes, one swizzle row
-constexpr int GSTAGES = 2;  // ring depth (two CTAs share an SM at N = 256)
+template <int BN>
+constexpr int GSTAGES = BN == 64 ? 4 : 2;  // ring depth (two CTAs share an SM at N = 256)
 constexpr int GTHREADS = 128;
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -91,11 +98,30 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                : "memory");
 }
 
-template <int BN>
+// NB products of one launch (parameters of the kernel).
+struct alignas(64) GemmOne {
+  CUtensorMap ta, tb;
+  float* C;
+  __nv_bfloat16 *Cb, *CbT;
+  const float* bias;
+  int M, N, K, ldc, ldcb, ldt, relu;
+};
+template <int NB>
+struct GemmSet {
+  GemmOne g[NB];
+};
+
+template <int BN, int NB>
 __global__ void __launch_bounds__(GTHREADS, 1)
-    k_gemm_tc(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, int M, int N, int K,
-              float* __restrict__ C, int ldc, __nv_bfloat16* __restrict__ Cb, int ldcb,
-              const float* __restrict__ bias, int relu, unsigned* __restrict__ err) {
+    k_gemm_tc(const __grid_constant__ GemmSet<NB> set, unsigned* __restrict__ err) {
+  const GemmOne& one = set.g[NB == 1 ? 0 : blockIdx.z];
+  const CUtensorMap &ta = one.ta, &tb = one.tb;
+  const int M = one.M, N = one.N, K = one.K, ldc = one.ldc, ldcb = one.ldcb, ldt = one.ldt, relu = one.relu;
+  float* __restrict__ C = one.C;
+  __nv_bfloat16 *__restrict__ Cb = one.Cb, *__restrict__ CbT = one.CbT;
+  const float* __restrict__ bias = one.bias;
+  const int m0 = blockIdx.x * GM, n0 = blockIdx.y * BN;
+  if (m0 >= M || n0 >= N) return;  // (products of one launch differ in size)
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "tcgen05 M = 128 takes N = 16 .. 256 in steps of 16");
   constexpr int TCOLS = BN < 32 ? 32 : BN;  // TMEM allocation: a power of two >= 32
   constexpr uint32_t A_BYTES = GM * GKC * 2, B_BYTES = BN * GKC * 2, STAGE = A_BYTES + B_BYTES;
@@ -104,14 +130,13 @@ __global__ void __launch_bounds__(GTHREADS, 1)
                              ((uint32_t)(GM >> 4) << 24);
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t full[GSTAGES], empty[GSTAGES], done;
+  __shared__ __align__(8) uint64_t full[GSTAGES<BN>], empty[GSTAGES<BN>], done;
   __shared__ uint32_t tmem_base;
   __shared__ int s_abort;
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.x * GM;
   const int nk = (K + GKC - 1) / GKC;
   if (tid == 0) {
-    for (int s = 0; s < GSTAGES; s++) {
+    for (int s = 0; s < GSTAGES<BN>; s++) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -133,8 +158,8 @@ __global__ void __launch_bounds__(GTHREADS, 1)
   if (w == 0 && lane == 0) {
     // producer: chunk kc into stage kc % GSTAGES once the MMAs of chunk kc - GSTAGES are done
     for (int kc = 0; kc < nk; kc++) {
-      const int s = kc % GSTAGES;
-      if (kc >= GSTAGES && !mbar_wait(&empty[s], ((kc / GSTAGES) + 1) & 1)) {
+      const int s = kc % GSTAGES<BN>;
+      if (kc >= GSTAGES<BN> && !mbar_wait(&empty[s], ((kc / GSTAGES<BN>) + 1) & 1)) {
         atomicOr(err, DEV_ERR_TIMEOUT);
         s_abort = 1;
         break;
@@ -143,14 +168,14 @@ __global__ void __launch_bounds__(GTHREADS, 1)
       unsigned char* a = sm + s * STAGE;
       mbar_expect_tx(&full[s], STAGE);
       tma_2d(a, &ta, kc * GKC, m0, &full[s]);
-      tma_2d(a + A_BYTES, &tb, kc * GKC, 0, &full[s]);
+      tma_2d(a + A_BYTES, &tb, kc * GKC, n0, &full[s]);
     }
   } else if (w == 1 && lane == 0) {
     // MMA issuer
     int kc = 0;
     for (; kc < nk; kc++) {
-      const int s = kc % GSTAGES;
-      if (!mbar_wait(&full[s], (kc / GSTAGES) & 1)) {
+      const int s = kc % GSTAGES<BN>;
+      if (!mbar_wait(&full[s], (kc / GSTAGES<BN>) & 1)) {
         atomicOr(err, DEV_ERR_TIMEOUT);
         s_abort = 1;
         break;
@@ -195,7 +220,7 @@ __global__ void __launch_bounds__(GTHREADS, 1)
 #pragma unroll
       for (int j = 0; j < 16; j++) stg[lane * 17 + j] = __uint_as_float(r[j]);
       __syncwarp();
-      const int n = c0 + cl;
+      const int n = n0 + c0 + cl;
       const float bn = (bias && n < N) ? bias[n] : 0.f;
 #pragma unroll 4
       for (int rr = 0; rr < 32; rr += 2) {
@@ -208,6 +233,16 @@ __global__ void __launch_bounds__(GTHREADS, 1)
           if (Cb) Cb[row * ldcb + n] = __float2bfloat16_rn(v);
         }
       }
+      if (CbT) {  // lanes are rows: 32 consecutive entries of a transposed row
+        const long long row = m0 + 32 * w + lane;
+#pragma unroll 4
+        for (int j = 0; j < 16; j++) {
+          const int nj = n0 + c0 + j;
+          float v = stg[lane * 17 + j] + ((bias && nj < N) ? bias[nj] : 0.f);
+          if (relu) v = fmaxf(v, 0.f);
+          if (row < M && nj < N) CbT[(long long)nj * ldt + row] = __float2bfloat16_rn(v);
+        }
+      }
       __syncwarp();
     }
   }
@@ -216,35 +251,67 @@ __global__ void __launch_bounds__(GTHREADS, 1)
   if (w == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS));
 }
 
-template <int BN>
-void launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, float* C, int ldc,
-                 __nv_bfloat16* Cb, int ldcb, const float* bias, bool relu, unsigned* err, cudaStream_t s) {
-  const size_t smem = (size_t)GSTAGES * (GM + BN) * GKC * 2 + 1024;
-  static bool attr[64] = {false};
+template <int BN, int NB>
+void launch_gemm(const GemmSet<NB>& set, dim3 grid, unsigned* err, cudaStream_t s) {
+  const size_t smem = (size_t)GSTAGES<BN> * (GM + BN) * GKC * 2 + 1024;
+  static std::atomic<bool> attr[64];  // per device: attribute set (idempotent, thread-safe)
   int dev = 0;
   PRBF_CUDA(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < 64 && !attr[dev]) {
-    PRBF_CUDA(cudaFuncSetAttribute(k_gemm_tc<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr[dev] = true;
+  if (dev < 0 || dev >= 64 || !attr[dev]) {
+    PRBF_CUDA(cudaFuncSetAttribute(k_gemm_tc<BN, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (dev >= 0 && dev < 64) attr[dev] = true;
   }
-  k_gemm_tc<BN><<<(M + GM - 1) / GM, GTHREADS, smem, s>>>(ta, tb, M, N, K, C, ldc, Cb, ldcb, bias, relu ? 1 : 0,
-                                                          err);
+  k_gemm_tc<BN, NB><<<grid, GTHREADS, smem, s>>>(set, err);
   PRBF_CHECK_LAUNCH();
+}
+
+GemmOne gemm_one(const GemmDesc& d, int bn) {
+  GemmOne g{};
+  g.ta = tile_map(d.A, d.M, d.K, d.lda, GM);
+  g.tb = tile_map(d.B, d.N, d.K, d.ldb, bn);
+  g.C = d.C;
+  g.Cb = d.Cb;
+  g.CbT = d.CbT;
+  g.bias = d.bias;
+  g.M = d.M;
+  g.N = d.N;
+  g.K = d.K;
+  g.ldc = d.ldc;
+  g.ldcb = d.ldcb;
+  g.ldt = d.ldt;
+  g.relu = d.relu ? 1 : 0;
+  return g;
 }
 
 }  // namespace
 
-void gemm_bf16_tc(int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, float* C,
-                  int ldc, __nv_bfloat16* Cb, int ldcb, const float* bias, bool relu, unsigned* err, cudaStream_t s) {
-  if (M <= 0 || N <= 0 || K <= 0) return;
-  if (N > 256) throw Error(PRBF_ERR_ARG, "GEMM N above 256");
-  if (N <= 16) {
-    const CUtensorMap ta = tile_map(A, M, K, lda, GM), tb = tile_map(B, N, K, ldb, 16);
-    launch_gemm<16>(ta, tb, M, N, K, C, ldc, Cb, ldcb, bias, relu, err, s);
+void gemm_bf16_tc(const GemmDesc& d, unsigned* err, cudaStream_t s) {
+  if (d.M <= 0 || d.N <= 0 || d.K <= 0) return;
+  if (d.N > 256) throw Error(PRBF_ERR_ARG, "GEMM N above 256");
+  const int mt = (d.M + GM - 1) / GM;
+  GemmSet<1> set;
+  if (d.N <= 16) {
+    set.g[0] = gemm_one(d, 16);
+    launch_gemm<16, 1>(set, dim3(mt), err, s);
+  } else if (mt < 76) {  // less than half an SM's share of row tiles: split the columns too
+    set.g[0] = gemm_one(d, 64);
+    launch_gemm<64, 1>(set, dim3(mt, (d.N + 63) / 64), err, s);
   } else {
-    const CUtensorMap ta = tile_map(A, M, K, lda, GM), tb = tile_map(B, N, K, ldb, 256);
-    launch_gemm<256>(ta, tb, M, N, K, C, ldc, Cb, ldcb, bias, relu, err, s);
+    set.g[0] = gemm_one(d, 256);
+    launch_gemm<256, 1>(set, dim3(mt), err, s);
   }
+}
+
+void gemm_bf16_tc_set(const GemmDesc (&d)[4], unsigned* err, cudaStream_t s) {
+  GemmSet<4> set;
+  int mt = 0, nt = 0;
+  for (int k = 0; k < 4; k++) {
+    if (d[k].M <= 0 || d[k].N <= 0 || d[k].K <= 0 || d[k].N > 256) throw Error(PRBF_ERR_ARG, "GEMM size");
+    set.g[k] = gemm_one(d[k], 64);
+    mt = std::max(mt, (d[k].M + GM - 1) / GM);
+    nt = std::max(nt, (d[k].N + 63) / 64);
+  }
+  launch_gemm<64, 4>(set, dim3(mt, nt, 4), err, s);
 }
 
 }  // namespace prbf

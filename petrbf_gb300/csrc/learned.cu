@@ -11,15 +11,6 @@
 namespace prbf {
 namespace {
 
-__global__ void k_gather_rows(const int* __restrict__ idx, int nb, const float* __restrict__ src, float* __restrict__ dst,
-                              int ncols) {
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < (long long)nb * ncols;
-       e += (long long)gridDim.x * blockDim.x) {
-    int r = (int)(e / ncols), k = (int)(e % ncols);
-    dst[e] = src[(long long)idx[r] * ncols + k];
-  }
-}
-
 uint64_t mix64(uint64_t& s) {
   uint64_t z = (s += 0x9E3779B97F4A7C15ull);
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -61,7 +52,7 @@ struct prbf_mlp {
   int device = 0;
   cudaStream_t stream = nullptr;
   Mlp net;
-  DevBuf<float> X, T, M, Xb, Tb, Mb, loss;
+  DevBuf<float> X, T, M, loss;
   DevBuf<int> idx;
   ~prbf_mlp() {
     if (stream) {
@@ -170,8 +161,8 @@ int prbf_mlp_loss_grad(prbf_mlp* m, int n, const float* X, const float* T, const
     upload_f(q.T, T, (size_t)n * MLP_OUT, q.stream);
     upload_f(q.M, M, (size_t)n * MLP_OUT, q.stream);
     PRBF_CUDA(cudaMemsetAsync(q.loss.get(), 0, sizeof(float), q.stream));
-    q.net.forward(q.X.get(), n, q.stream);
-    q.net.backward(q.X.get(), q.T.get(), q.M.get(), n, (float)(1.0 / cnt), q.loss.get(), q.stream);
+    q.net.forward(q.X.get(), n, q.stream, true);
+    q.net.backward(q.T.get(), q.M.get(), n, (float)(1.0 / cnt), q.loss.get(), q.stream);
     if (loss) PRBF_CUDA(cudaMemcpyAsync(loss, q.loss.get(), sizeof(float), cudaMemcpyDeviceToHost, q.stream));
     if (grad_out)
       PRBF_CUDA(cudaMemcpyAsync(grad_out, q.net.grad.get(), sizeof(float) * mlp_param_count(), cudaMemcpyDeviceToHost,
@@ -194,9 +185,6 @@ int prbf_mlp_train(prbf_mlp* m, int n, const float* X, const float* T, const flo
       for (int j = 0; j < MLP_OUT; j++) c += M[(size_t)r * MLP_OUT + j];
       rowcnt[r] = c;
     }
-    q.Xb.reserve((size_t)batch * MLP_IN);
-    q.Tb.reserve((size_t)batch * MLP_OUT);
-    q.Mb.reserve((size_t)batch * MLP_OUT);
     q.idx.reserve(n);
     std::vector<int> perm(n);
     uint64_t rs = seed;
@@ -212,12 +200,8 @@ int prbf_mlp_train(prbf_mlp* m, int n, const float* X, const float* T, const flo
         for (int r = b0; r < b0 + nb; r++) cnt += rowcnt[perm[r]];
         if (cnt <= 0) continue;
         const int* id = q.idx.get() + b0;
-        k_gather_rows<<<256, 256, 0, s>>>(id, nb, q.X.get(), q.Xb.get(), MLP_IN);
-        k_gather_rows<<<64, 256, 0, s>>>(id, nb, q.T.get(), q.Tb.get(), MLP_OUT);
-        k_gather_rows<<<64, 256, 0, s>>>(id, nb, q.M.get(), q.Mb.get(), MLP_OUT);
-        PRBF_CHECK_LAUNCH();
-        q.net.forward(q.Xb.get(), nb, s);
-        q.net.backward(q.Xb.get(), q.Tb.get(), q.Mb.get(), nb, (float)(1.0 / cnt), q.loss.get(), s);
+        q.net.forward(q.X.get(), nb, s, true, id);
+        q.net.backward(q.T.get(), q.M.get(), nb, (float)(1.0 / cnt), q.loss.get(), s, id);
         q.net.adam(lr, s);
         nbatch++;
       }

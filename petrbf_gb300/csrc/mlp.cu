@@ -29,37 +29,103 @@
 namespace prbf {
 namespace {
 
-// dY = 2 mask (Y - T) / sum(mask); loss partial sums
-__global__ void k_mse(int n, const float* __restrict__ Y, const float* __restrict__ T, const float* __restrict__ Msk,
-                      float inv_cnt, float* __restrict__ dY, float* __restrict__ loss) {
-  float l = 0.f;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float d = (Y[i] - T[i]) * Msk[i];
-    dY[i] = 2.f * d * inv_cnt;
-    l += d * d;
+// A training step of 512 rows is a chain of small kernels, so what counts is their number and
+// the time from one to the next: 14 launches (the rows gathered, converted and transposed in one,
+// four products forward, for each layer the gradient's mask, conversion, transpose and bias sum in
+// one and a product back, all four weight gradients in one, Adam with the weights' BF16 copies in
+// one) where there were 41: 0.39 -> 0.16 ms a step.
+
+// X rows (or rows idx[.] of it) as BF16, and transposed [K][ldn]: 32 x 32 tiles through shared
+// memory, 32 x 8 threads. K a multiple of 32.
+__global__ void k_pack_rows(int n, int K, const int* __restrict__ idx, const float* __restrict__ X,
+                            __nv_bfloat16* __restrict__ Xb, __nv_bfloat16* __restrict__ XT, int ldn) {
+  __shared__ __nv_bfloat16 t[32][33];
+  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+  for (int k = threadIdx.y; k < 32; k += 8) {
+    const int r = r0 + k, c = c0 + threadIdx.x;
+    if (r < n) {
+      const __nv_bfloat16 v = __float2bfloat16_rn(X[(long long)(idx ? idx[r] : r) * K + c]);
+      Xb[(long long)r * K + c] = v;
+      t[k][threadIdx.x] = v;
+    }
   }
-  l = warp_sum(l);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, l * inv_cnt);
+  __syncthreads();
+  for (int k = threadIdx.y; k < 32; k += 8) {
+    const int r = r0 + threadIdx.x;
+    if (r < n) XT[(long long)(c0 + k) * ldn + r] = t[threadIdx.x][k];
+  }
 }
 
-// dZ = dH * (H > 0)
-__global__ void k_relu_back(int n, const float* __restrict__ H, float* __restrict__ dH) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    if (!(H[i] > 0.f)) dH[i] = 0.f;
+// The gradient dZ of a layer's output before its ReLU, as the two GEMM operands (BF16, row-major
+// and transposed [N][ldn]) and its column sums db (FP32, rows added in order). LOSS: dZ = 2 mask
+// (Y - T) / sum(mask) from the output Y and the targets and masks of rows idx[.], and the loss;
+// otherwise dZ = dH where the layer's output H is positive. One CTA per 32 columns walks the rows
+// 128 at a time, 32 x 32 threads; its first warp adds the rows while the others fetch the next.
+template <bool LOSS>
+__global__ void __launch_bounds__(1024) k_back_prep(int n, int N, const float* __restrict__ Yd,
+                                                    const float* __restrict__ H, const float* __restrict__ T,
+                                                    const float* __restrict__ Msk, const int* __restrict__ idx,
+                                                    float inv_cnt, __nv_bfloat16* __restrict__ dzb,
+                                                    __nv_bfloat16* __restrict__ dzT, int ldn, float* __restrict__ db,
+                                                    float* __restrict__ loss) {
+  constexpr int R = 4, TR = 32 * R;  // rows per thread and per tile
+  __shared__ float t[2][TR][33];
+  const int tx = threadIdx.x, ty = threadIdx.y, c = blockIdx.x * 32 + tx;
+  float sum = 0.f, l = 0.f, v[R];
+  auto fetch = [&](int r0) {
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+      const int r = r0 + 32 * k + ty;
+      v[k] = 0.f;
+      if (r < n && c < N) {
+        const long long e = (long long)r * N + c;
+        if constexpr (LOSS) {
+          const long long q = idx ? (long long)idx[r] * N + c : e;
+          const float d = (Yd[e] - T[q]) * Msk[q];
+          v[k] = 2.f * d * inv_cnt;
+          l += d * d;
+        } else {
+          v[k] = H[e] > 0.f ? Yd[e] : 0.f;
+        }
+      }
+    }
+  };
+  fetch(0);
+  for (int r0 = 0, b = 0; r0 < n; r0 += TR, b ^= 1) {
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+      const int r = r0 + 32 * k + ty;
+      t[b][32 * k + ty][tx] = v[k];
+      if (dzb && r < n && c < N) dzb[(long long)r * N + c] = __float2bfloat16_rn(v[k]);
+    }
+    if (r0 + TR < n) fetch(r0 + TR);
+    __syncthreads();
+    const int ct = blockIdx.x * 32 + ty;  // transposed: this warp's column, lanes rows
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+      const int rt = r0 + 32 * k + tx;
+      if (rt < n && ct < N) dzT[(long long)ct * ldn + rt] = __float2bfloat16_rn(t[b][32 * k + tx][ty]);
+    }
+    if (ty == 0) {
+      const int m = min(TR, n - r0);
+#pragma unroll 16
+      for (int k = 0; k < m; k++) sum += t[b][k][tx];
+    }
+  }
+  if (ty == 0 && c < N) db[c] = sum;
+  if constexpr (LOSS) {
+    l = warp_sum(l);
+    if (tx == 0) atomicAdd(loss, l * inv_cnt);
+  }
 }
 
-// db[j] = sum_m dZ[m][j]
-__global__ void k_colsum(int M, int N, const float* __restrict__ dZ, float* __restrict__ db) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= N) return;
-  float s = 0.f;
-  for (int m = 0; m < M; m++) s += dZ[(long long)m * N + j];
-  db[j] = s;
-}
-
+// Adam, and the weights' BF16 copies: row-major, and each layer's matrix transposed. The layers
+// are [256][256] weights and 256 biases but the last, [16][256] and 16.
 __global__ void k_adam(int n, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m1,
-                       float* __restrict__ m2, __nv_bfloat16* __restrict__ wb, float lr, float b1, float b2, float c1,
-                       float c2, float eps) {
+                       float* __restrict__ m2, __nv_bfloat16* __restrict__ wb, __nv_bfloat16* __restrict__ wbT,
+                       float lr, float b1, float b2, float c1, float c2, float eps) {
+  constexpr int LAYER = MLP_HID * MLP_IN + MLP_HID;
+  static_assert(MLP_IN == MLP_HID, "equal hidden layers");
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     float gi = g[i];
     float a = b1 * m1[i] + (1.f - b1) * gi;
@@ -68,7 +134,11 @@ __global__ void k_adam(int n, float* __restrict__ w, const float* __restrict__ g
     m2[i] = b;
     float wi = w[i] - lr * (a * c1) / (sqrtf(b * c2) + eps);
     w[i] = wi;
-    if (wb) wb[i] = __float2bfloat16_rn(wi);
+    const __nv_bfloat16 q = __float2bfloat16_rn(wi);
+    wb[i] = q;
+    const int l = min(i / LAYER, MLP_LAYERS - 1), o = l * LAYER, e = i - o;
+    const int N = l < MLP_LAYERS - 1 ? MLP_HID : MLP_OUT;
+    if (e < N * MLP_IN) wbT[o + (e % MLP_IN) * N + e / MLP_IN] = q;
   }
 }
 
@@ -278,69 +348,90 @@ size_t Mlp::woff(int l) const {
 }
 
 // Forward for n rows of X (device); the activations (FP32, and BF16 as the next GEMM's
-// operand) are kept for the backward pass.
-void Mlp::forward(const float* X, int n, cudaStream_t s) {
+// operand) are kept, for training also their transposes, the weight gradients' operands.
+void Mlp::forward(const float* X, int n, cudaStream_t s, bool train, const int* idx) {
   xb.reserve((size_t)n * MLP_IN);
-  to_bf16((long long)n * MLP_IN, X, xb.get(), s);
-  const __nv_bfloat16* in = xb.get();
+  const int ldn = (n + 7) / 8 * 8;  // transposed operands: rows padded to 16 bytes
+  if (train) {
+    for (int l = 0; l < MLP_LAYERS; l++) hT[l].reserve((size_t)MLP_HID * ldn);
+    k_pack_rows<<<dim3(MLP_IN / 32, (n + 31) / 32), dim3(32, 8), 0, s>>>(n, MLP_IN, idx, X, xb.get(), hT[0].get(), ldn);
+    PRBF_CHECK_LAUNCH();
+  } else {
+    to_bf16((long long)n * MLP_IN, X, xb.get(), s);
+  }
   for (int l = 0; l < MLP_LAYERS; l++) {
     acts[l].reserve((size_t)n * kLayerOut[l]);
     const bool hidden = l < MLP_LAYERS - 1;
     if (hidden) actb[l].reserve((size_t)n * kLayerOut[l]);
     const size_t o = woff(l);
-    const float* b = w.get() + o + (size_t)kLayerIn[l] * kLayerOut[l];
-    gemm_bf16_tc(n, kLayerOut[l], kLayerIn[l], in, kLayerIn[l], wb.get() + o, kLayerIn[l], acts[l].get(),
-                 kLayerOut[l], hidden ? actb[l].get() : nullptr, kLayerOut[l], b, hidden, err.get(), s);
-    if (hidden) in = actb[l].get();
+    GemmDesc d;
+    d.M = n;
+    d.N = d.ldc = d.ldcb = kLayerOut[l];
+    d.K = d.lda = d.ldb = kLayerIn[l];
+    d.A = l ? actb[l - 1].get() : xb.get();
+    d.B = wb.get() + o;
+    d.C = acts[l].get();
+    d.Cb = hidden ? actb[l].get() : nullptr;
+    if (train && hidden) {
+      d.CbT = hT[l + 1].get();
+      d.ldt = ldn;
+    }
+    d.bias = w.get() + o + (size_t)kLayerIn[l] * kLayerOut[l];
+    d.relu = hidden;
+    gemm_bf16_tc(d, err.get(), s);
   }
 }
 
-// Loss and gradients (into grad) for n rows; returns nothing, loss accumulated on device.
-void Mlp::backward(const float* X, const float* T, const float* Msk, int n, float inv_cnt, float* dloss,
-                   cudaStream_t s) {
-  size_t np = mlp_param_count();
-  dact[0].reserve((size_t)n * MLP_HID);
-  dact[1].reserve((size_t)n * MLP_HID);
-  float* dY = dact[0].get();
-  k_mse<<<256, 256, 0, s>>>(n * MLP_OUT, acts[MLP_LAYERS - 1].get(), T, Msk, inv_cnt, dY, dloss);
-  PRBF_CHECK_LAUNCH();
-  (void)np;
-  (void)X;  // its BF16 copy from the forward pass is the first layer's operand
-  const int ldn = (n + 7) / 8 * 8;  // transposed operands: rows padded to 16 bytes
+// Gradients (into grad) of the n rows of the last training forward pass; loss accumulated on
+// the device.
+void Mlp::backward(const float* T, const float* Msk, int n, float inv_cnt, float* dloss, cudaStream_t s,
+                   const int* idx) {
+  dact.reserve((size_t)n * MLP_HID);
+  const int ldn = (n + 7) / 8 * 8;
   dzb.reserve((size_t)n * MLP_HID);
-  dzT.reserve((size_t)MLP_HID * ldn);
-  hT.reserve((size_t)MLP_HID * ldn);
-  float* dcur = dY;
+  GemmDesc dw[MLP_LAYERS];
   for (int l = MLP_LAYERS - 1; l >= 0; l--) {
     const int K = kLayerIn[l], N = kLayerOut[l];
-    const __nv_bfloat16* Hin = l > 0 ? actb[l - 1].get() : xb.get();
-    size_t o = woff(l);
-    to_bf16((long long)n * N, dcur, dzb.get(), s);
-    transpose_bf16(n, N, dzb.get(), N, dzT.get(), ldn, s);
-    transpose_bf16(n, K, Hin, K, hT.get(), ldn, s);
-    // dW[N][K] = dZ^T Hin (the batch is the inner dimension) ; db = colsum dZ (FP32)
-    gemm_bf16_tc(N, K, n, dzT.get(), ldn, hT.get(), ldn, grad.get() + o, K, nullptr, 0, nullptr, false, err.get(), s);
-    k_colsum<<<(N + 127) / 128, 128, 0, s>>>(n, N, dcur, grad.get() + o + (size_t)K * N);
+    const size_t o = woff(l);
+    dzT[l].reserve((size_t)N * ldn);
+    float* db = grad.get() + o + (size_t)K * N;
+    const dim3 grid((N + 31) / 32), block(32, 32);
+    if (l == MLP_LAYERS - 1)
+      k_back_prep<true><<<grid, block, 0, s>>>(n, N, acts[l].get(), nullptr, T, Msk, idx, inv_cnt, dzb.get(),
+                                               dzT[l].get(), ldn, db, dloss);
+    else
+      k_back_prep<false><<<grid, block, 0, s>>>(n, N, dact.get(), acts[l].get(), nullptr, nullptr, nullptr, 0.f,
+                                                l ? dzb.get() : nullptr, dzT[l].get(), ldn, db, nullptr);
     PRBF_CHECK_LAUNCH();
-    if (l > 0) {
-      float* dprev = dact[(MLP_LAYERS - l) & 1].get();
-      // dH[n][K] = dZ W, W^T [K][N] as the K-major operand
-      gemm_bf16_tc(n, K, N, dzb.get(), N, wbT.get() + o, N, dprev, K, nullptr, 0, nullptr, false, err.get(), s);
-      k_relu_back<<<256, 256, 0, s>>>(n * K, acts[l - 1].get(), dprev);
-      PRBF_CHECK_LAUNCH();
-      dcur = dprev;
+    // dW[N][K] = dZ^T Hin (the batch is the inner dimension)
+    dw[l].M = N;
+    dw[l].N = dw[l].ldc = K;
+    dw[l].K = n;
+    dw[l].A = dzT[l].get();
+    dw[l].B = hT[l].get();
+    dw[l].lda = dw[l].ldb = ldn;
+    dw[l].C = grad.get() + o;
+    if (l > 0) {  // dH[n][K] = dZ W, W^T [K][N] as the K-major operand
+      GemmDesc d;
+      d.M = n;
+      d.N = d.ldc = K;
+      d.K = d.lda = d.ldb = N;
+      d.A = dzb.get();
+      d.B = wbT.get() + o;
+      d.C = dact.get();
+      gemm_bf16_tc(d, err.get(), s);
     }
   }
+  gemm_bf16_tc_set(dw, err.get(), s);
 }
 
 void Mlp::adam(float lr, cudaStream_t s) {
   step++;
   const float b1 = 0.9f, b2 = 0.999f;
   float c1 = 1.f / (1.f - std::pow(b1, (float)step)), c2 = 1.f / (1.f - std::pow(b2, (float)step));
-  k_adam<<<256, 256, 0, s>>>((int)mlp_param_count(), w.get(), grad.get(), m1.get(), m2.get(), nullptr, lr, b1, b2, c1,
-                             c2, 1e-8f);
+  k_adam<<<256, 256, 0, s>>>((int)mlp_param_count(), w.get(), grad.get(), m1.get(), m2.get(), wb.get(), wbT.get(), lr,
+                             b1, b2, c1, c2, 1e-8f);
   PRBF_CHECK_LAUNCH();
-  refresh_bf16(s);
 }
 
 int fine_cells(Ctx& c, PointSet& P, Workspace& ws, DevBuf<int>& cells) {

@@ -25,16 +25,21 @@ struct Mlp {
   DevBuf<float> w, grad, m1, m2;
   DevBuf<__nv_bfloat16> wb, wbT;
   DevBuf<float> acts[MLP_LAYERS];
-  DevBuf<float> dact[2];
-  DevBuf<__nv_bfloat16> xb, actb[MLP_LAYERS - 1], dzb, dzT, hT;
+  DevBuf<float> dact;  // gradient of a layer's input, before the ReLU below
+  // GEMM operands in BF16: the inputs and activations, for training also transposed (hT[l]: the
+  // input of layer l), and the output gradients (dzT[l]: transposed, of layer l)
+  DevBuf<__nv_bfloat16> xb, actb[MLP_LAYERS - 1], dzb, hT[MLP_LAYERS], dzT[MLP_LAYERS];
   DevBuf<unsigned> err;
   int step = 0;
   bool ready = false;
   void init(uint64_t seed, cudaStream_t s);
   void set_weights(const float* host, cudaStream_t s);
   size_t woff(int l) const;
-  void forward(const float* X, int n, cudaStream_t s);
-  void backward(const float* X, const float* T, const float* Msk, int n, float inv_cnt, float* dloss, cudaStream_t s);
+  // n rows of X (of rows idx[0 .. n) when idx is given); train: also what backward needs
+  void forward(const float* X, int n, cudaStream_t s, bool train = false, const int* idx = nullptr);
+  // gradients of the rows of the last training forward pass (targets and masks of the same rows)
+  void backward(const float* T, const float* Msk, int n, float inv_cnt, float* dloss, cudaStream_t s,
+                const int* idx = nullptr);
   void adam(float lr, cudaStream_t s);
   // raises PRBF_ERR_TIMEOUT if a GEMM's bounded wait gave up since the last check (syncs s)
   void check(cudaStream_t s);
@@ -46,10 +51,26 @@ struct Mlp {
 
 // C[M][N] = A[M][K] B[N][K]^T (+ bias, ReLU) on the tensor cores (gemm_tc.cu): A and B
 // BF16 row-major with K contiguous (leading dimensions lda, ldb multiples of 8, 16-byte
-// aligned bases), FP32 accumulation; C (FP32, ldc) and/or Cb (BF16, ldcb) may be null.
-// N <= 256; entries past the matrix edges read as zero.
-void gemm_bf16_tc(int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, float* C,
-                  int ldc, __nv_bfloat16* Cb, int ldcb, const float* bias, bool relu, unsigned* err, cudaStream_t s);
+// aligned bases), FP32 accumulation; C (FP32, ldc), Cb (BF16, ldcb) and CbT (BF16, transposed
+// [N][ldt]) may be null. N <= 256; entries past the matrix edges read as zero.
+struct GemmDesc {
+  int M = 0, N = 0, K = 0;
+  const __nv_bfloat16* A = nullptr;
+  int lda = 0;
+  const __nv_bfloat16* B = nullptr;
+  int ldb = 0;
+  float* C = nullptr;
+  int ldc = 0;
+  __nv_bfloat16* Cb = nullptr;
+  int ldcb = 0;
+  __nv_bfloat16* CbT = nullptr;
+  int ldt = 0;
+  const float* bias = nullptr;
+  bool relu = false;
+};
+void gemm_bf16_tc(const GemmDesc& d, unsigned* err, cudaStream_t s);
+// Four products in one launch.
+void gemm_bf16_tc_set(const GemmDesc (&d)[4], unsigned* err, cudaStream_t s);
 
 // Non-empty fine cells of P (compacted list), returns their count.
 int fine_cells(Ctx& c, PointSet& P, Workspace& ws, DevBuf<int>& cells);
