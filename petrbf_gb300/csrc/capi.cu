@@ -45,8 +45,11 @@ Grid make_grid(int dim, const double* b, double sigma, int nsigma_box, int sigma
 }
 
 void ctx_stream_release(Ctx& c) {
-  if (c.stream) cudaStreamSynchronize(c.stream);
-  if (c.stream) cudaStreamDestroy(c.stream);
+  if (c.stream) {
+    cudaStreamSynchronize(c.stream);
+    dev_pool_stream_done(c.device, c.stream);
+    cudaStreamDestroy(c.stream);
+  }
   c.stream = nullptr;
 }
 
@@ -188,11 +191,12 @@ int prbf_ctx_create(const prbf_params* p, prbf_ctx** out) {
     if (p->device < 0 || p->device >= ndev) throw Error(PRBF_ERR_ARG, "no such CUDA device");
     PRBF_CUDA(cudaSetDevice(p->device));
     PRBF_CUDA(cudaStreamCreateWithFlags(&ctx->c.stream, cudaStreamNonBlocking));
+    StreamScope scope(ctx->c.stream);
     ctx->c.err.reserve(4);
     PRBF_CUDA(cudaMemsetAsync(ctx->c.err.get(), 0, 16, ctx->c.stream));
   } catch (const Error& e) {
     int st = e.status;
-    delete ctx;
+    delete ctx;  // (outside of any scope: its buffers are freed)
     return st;
   }
   *out = ctx;
@@ -202,6 +206,9 @@ int prbf_ctx_create(const prbf_params* p, prbf_ctx** out) {
 int prbf_ctx_destroy(prbf_ctx* ctx) {
   if (!ctx) return PRBF_ERR_ARG;
   cudaSetDevice(ctx->c.device);
+  // every buffer is idle once the stream is: ~Ctx waits for it before it frees the first
+  if (ctx->c.stream) cudaStreamSynchronize(ctx->c.stream);
+  StreamScope scope(ctx->c.stream, true);
   delete ctx;
   return PRBF_OK;
 }

@@ -78,6 +78,7 @@ int ctx_call(prbf_ctx* ctx, F&& f) {
   try {
     c.last_error.clear();
     PRBF_CUDA(cudaSetDevice(c.device));
+    StreamScope scope(c.stream);
     f(c);
     return PRBF_OK;
   } catch (const Error& e) {

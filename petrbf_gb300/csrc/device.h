@@ -10,7 +10,27 @@
 
 namespace prbf {
 
-// Owning device buffer (cudaMalloc / cudaFree), grow-only.
+// ---- devpool.cu --------------------------------------------------------------------
+// Device memory kept between uses. Inside a StreamScope (a call on a context) freed blocks are
+// kept for the scope's stream; idle: the stream has no work left, any stream may take them.
+struct StreamScope {
+  StreamScope(cudaStream_t s, bool idle = false);
+  ~StreamScope();
+  StreamScope(const StreamScope&) = delete;
+  StreamScope& operator=(const StreamScope&) = delete;
+
+ private:
+  cudaStream_t stream;
+  bool on, was_idle;
+};
+cudaError_t dev_alloc(void** p, size_t bytes);
+void dev_free(void* p);
+// The stream is idle and about to be destroyed: its blocks may serve others.
+void dev_pool_stream_done(int device, cudaStream_t s);
+// Gives the current device's kept blocks back to the driver.
+void dev_pool_trim();
+
+// Owning device buffer, grow-only.
 template <class T>
 struct DevBuf {
   T* p = nullptr;
@@ -20,7 +40,7 @@ struct DevBuf {
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() { release(); }
   void release() {
-    if (p) cudaFree(p);
+    if (p) dev_free(p);
     p = nullptr;
     n = 0;
   }
@@ -30,7 +50,7 @@ struct DevBuf {
     release();
     size_t bytes = count * sizeof(T);
     if (bytes == 0) bytes = 16;
-    const cudaError_t e = cudaMalloc((void**)&p, bytes);
+    const cudaError_t e = dev_alloc((void**)&p, bytes);
     if (e != cudaSuccess) {
       p = nullptr;
       cudaGetLastError();  // an allocation failure is not sticky: later launch checks must not see it
