@@ -61,6 +61,14 @@ struct SegSkip {
   __device__ bool cell_done(int c) const { return done && done[(long long)cprob[c] * stride]; }
 };
 
+// Several vectors (right-hand sides) whose systems stop one by one: done[v * stride] of the nv
+// vectors of a launch; inactive when done is null. A kernel of NV vectors is launched for every
+// count up to nv and runs when that many are left, on those (vec_map); the others return.
+struct VecSkip {
+  const int* done = nullptr;
+  int stride = 0, nv = 0;
+};
+
 __host__ __device__ inline int cell_of(const Grid& g, int ix, int iy, int iz) {
   return g.dim == 2 ? ix * g.ny + iy : (iz * g.nx + ix) * g.ny + iy;
 }
@@ -84,6 +92,23 @@ __host__ __device__ inline void cell_xyz(const Grid& g, int ic, int& ix, int& iy
 // bit-identical to the unfused host/CPU evaluation (2d/get_cluster.h:217-218).
 __device__ __forceinline__ double centre_coord(double lo, int i, double box) {
   return __dadd_rn(lo, __dmul_rn((double)i + 0.5, box));
+}
+
+template <int NV>
+__device__ __forceinline__ bool vec_map(const VecSkip& k, int (&map)[NV]) {
+#pragma unroll
+  for (int q = 0; q < NV; q++) map[q] = q;
+  if (!k.done) return true;
+  int left = 0;
+#pragma unroll
+  for (int v = 0; v < 4; v++)
+    if (v < k.nv && !k.done[(long long)v * k.stride]) {
+#pragma unroll
+      for (int q = 0; q < NV; q++)
+        if (q == left) map[q] = v;
+      left++;
+    }
+  return left == NV;
 }
 
 // ---- TMA bulk copies (cp.async.bulk, non-tensor) and mbarriers -------------------------

@@ -169,10 +169,22 @@ bool gauss_plan_sym_batch(GaussPlan& plan, const std::vector<Grid>& grids, const
                           const std::vector<int>& hcs, cudaStream_t s);
 // w[i] = sum_{j in trunc(cell(i))} g[j] exp(-|t_i - s_j|^2 / (2 sigma^2)) / (2 pi sigma^2)
 // for all sorted targets i; g must be a padded device vector of src.n (+2) entries.
-// w = A g for nv weight vectors at stride vstride (even; vectors padded as the sources)
+// w = A g for nv weight vectors at stride vstride (even; vectors padded as the sources);
+// left: those of stopped systems left out (the kernels that take several vectors)
 void gauss_sum_dev(const GaussPlan& plan, const PointsView& tgt, const PointsView& src,
                    const double* g, double* w, bool fp32, unsigned* err, cudaStream_t s,
-                   const int* skip = nullptr, int nv = 1, long long vstride = 0);
+                   const int* skip = nullptr, int nv = 1, long long vstride = 0, VecSkip left = VecSkip{});
+// Launches f(k), a launch of k vectors, for every count of vectors that may be left of nv.
+template <class F>
+inline void for_counts(const VecSkip& left, int nv, F&& f) {
+  for (int k = left.done ? 1 : nv; k <= nv; k++) f(k);
+}
+// Of the vectors v0 .. v0 + nv - 1.
+inline VecSkip vec_part(VecSkip left, int v0, int nv) {
+  if (left.done) left.done += (long long)v0 * left.stride;
+  left.nv = nv;
+  return left;
+}
 
 // Device address of the FP64 exponential table of the sums (n = 1024 entries of the
 // T[j]-folded cubic, 4 coefficients each), uploaded to the current device on first use.

@@ -533,8 +533,10 @@ __global__ void __launch_bounds__(kThreads, 6) k_gauss_f32m(
     const double* __restrict__ tz, const int* __restrict__ cs_t, const float* __restrict__ su,
     const float* __restrict__ sv, const float* __restrict__ sw, const unsigned long long* __restrict__ smask,
     const float* __restrict__ sg, long long vs_g, const int* __restrict__ cs_s, double* __restrict__ w,
-    long long vs_w, double scale0, double norm0, unsigned* err, const int* __restrict__ skip) {
+    long long vs_w, double scale0, double norm0, unsigned* err, const int* __restrict__ skip, VecSkip left) {
   if (skip && *skip) return;
+  int vm[NV];
+  if (!vec_map<NV>(left, vm)) return;
   using Lay = LayoutF<DIM, NV>;
   constexpr int NF = Lay::NF, RC = Lay::RC, NX = Lay::NX;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -737,7 +739,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_gauss_f32m(
             bulk_g2s(rawf + RC + dst, sv + s_al, len * 4u, bar);
             if (DIM == 3) bulk_g2s(rawf + 2 * RC + dst, sw + s_al, len * 4u, bar);
 #pragma unroll
-            for (int v = 0; v < NV; v++) bulk_g2s(rawf + (DIM + v) * RC + dst, sg + v * vs_g + s_al, len * 4u, bar);
+            for (int v = 0; v < NV; v++) bulk_g2s(rawf + (DIM + v) * RC + dst, sg + vm[v] * vs_g + s_al, len * 4u, bar);
             bulk_g2s(rawm + dst, smask + s_al, len * 8u, bar);
           }
         }
@@ -819,7 +821,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_gauss_f32m(
     for (int t = tid; t < nt; t += kThreads)
 #pragma unroll
       for (int v = 0; v < NV; v++)
-        w[v * vs_w + t0 + t] = (double)acc[v * kTileT + t] * norm;
+        w[vm[v] * vs_w + t0 + t] = (double)acc[v * kTileT + t] * norm;
   }
 }
 
@@ -1538,9 +1540,16 @@ void launch_sym_nv(const GaussPlan& P, const PointsView& s, const double* gv, do
   }
 }
 
+// FP32 copies of nv weight vectors
+void convert_f32(const GaussPlan& P, int n, int nv, const double* gv, long long vstride, const int* skip,
+                 cudaStream_t st) {
+  k_to_f32<<<4 * 152, 256, 0, st>>>(n, nv, vstride, P.g32_stride, gv, P.g32.get(), skip);
+  PRBF_CHECK_LAUNCH();
+}
+
 template <int DIM, int NV, bool BATCH>
 void launch_f32m(const GaussPlan& P, const PointsView& t, const PointsView& s, const double* gv, double* w,
-                 long long vstride, unsigned* err, const int* skip, cudaStream_t st) {
+                 long long vstride, unsigned* err, const int* skip, cudaStream_t st, VecSkip left = VecSkip{}) {
   constexpr size_t sm = LayoutF<DIM, NV>::total;
   static_assert(sm <= 227 * 1024, "k_gauss_f32m shared memory");
   static std::atomic<bool> attr_set[64];  // per device: attribute set (idempotent, thread-safe)
@@ -1552,34 +1561,39 @@ void launch_f32m(const GaussPlan& P, const PointsView& t, const PointsView& s, c
     if (dev < 64) attr_set[dev] = true;
   }
   const SumConsts k0 = sum_consts(P.g.sigma, true, 0);
-  k_to_f32<<<4 * 152, 256, 0, st>>>(s.n, NV, vstride, P.g32_stride, gv, P.g32.get(), skip);
-  PRBF_CHECK_LAUNCH();
   const int grid = P.grid > 0 ? std::min(P.grid, P.nitems) : P.nitems;
   k_gauss_f32m<DIM, NV, BATCH><<<grid, kThreads, sm, st>>>(
       P.g, P.grids.get(), P.cprob.get(), P.seg, P.items.get(), P.nitems, t.x, t.y, t.z, t.cell_start, P.su.get(),
       P.sv.get(), P.sw.get(), P.smask.get(), P.g32.get(), P.g32_stride, s.cell_start, w, vstride, k0.scale, k0.norm,
-      err, skip);
+      err, skip, left);
   PRBF_CHECK_LAUNCH();
 }
 
 template <int DIM, bool F32>
 void launch_nv(const GaussPlan& P, const PointsView& t, const PointsView& s, const double* gv, double* w, int nv,
-               long long vstride, unsigned* err, const int* skip, cudaStream_t st) {
+               long long vstride, unsigned* err, const int* skip, VecSkip left, cudaStream_t st) {
   if (F32 && P.f32_ready && P.batched) {
-    for (int v = 0; v < nv; v++)
+    for (int v = 0; v < nv; v++) {
+      convert_f32(P, s.n, 1, gv + v * vstride, vstride, skip, st);
       launch_f32m<DIM, 1, true>(P, t, s, gv + v * vstride, w + v * vstride, vstride, err, skip, st);
+    }
     return;
   }
   if (F32 && P.f32_ready) {
     for (int v0 = 0; v0 < nv; v0 += 4) {
       const double* g0 = gv + v0 * vstride;
       double* w0 = w + v0 * vstride;
-      switch (std::min(4, nv - v0)) {
-        case 1: launch_f32m<DIM, 1, false>(P, t, s, g0, w0, vstride, err, skip, st); break;
-        case 2: launch_f32m<DIM, 2, false>(P, t, s, g0, w0, vstride, err, skip, st); break;
-        case 3: launch_f32m<DIM, 3, false>(P, t, s, g0, w0, vstride, err, skip, st); break;
-        default: launch_f32m<DIM, 4, false>(P, t, s, g0, w0, vstride, err, skip, st); break;
-      }
+      const int k0 = std::min(4, nv - v0);
+      const VecSkip l0 = vec_part(left, v0, k0);
+      convert_f32(P, s.n, k0, g0, vstride, skip, st);
+      for_counts(l0, k0, [&](int k) {
+        switch (k) {
+          case 1: launch_f32m<DIM, 1, false>(P, t, s, g0, w0, vstride, err, skip, st, l0); break;
+          case 2: launch_f32m<DIM, 2, false>(P, t, s, g0, w0, vstride, err, skip, st, l0); break;
+          case 3: launch_f32m<DIM, 3, false>(P, t, s, g0, w0, vstride, err, skip, st, l0); break;
+          default: launch_f32m<DIM, 4, false>(P, t, s, g0, w0, vstride, err, skip, st, l0); break;
+        }
+      });
     }
     return;
   }
@@ -1816,7 +1830,7 @@ void gauss_plan_forms_batch(GaussPlan& plan, const std::vector<Grid>& grids, con
 
 void gauss_sum_dev(const GaussPlan& P, const PointsView& t, const PointsView& s, const double* gv,
                    double* w, bool fp32, unsigned* err, cudaStream_t st, const int* skip, int nv,
-                   long long vstride) {
+                   long long vstride, VecSkip left) {
   if (P.nitems == 0 || nv <= 0) return;
   if (nv > 1 && (vstride % 2 || vstride < t.n || vstride < s.n))
     throw Error(PRBF_ERR_ARG, "vector stride must be even and cover the points");
@@ -1832,19 +1846,19 @@ void gauss_sum_dev(const GaussPlan& P, const PointsView& t, const PointsView& s,
     return;
   }
   if (!fp32 && P.fx_ready && !P.pipe64) {
-    gauss_fx_sum(P, t, s, gv, w, err, skip, nv, vstride, st);
+    gauss_fx_sum(P, t, s, gv, w, err, skip, nv, vstride, left, st);
     return;
   }
   if (P.g.dim == 2) {
     if (fp32)
-      launch_nv<2, true>(P, t, s, gv, w, nv, vstride, err, skip, st);
+      launch_nv<2, true>(P, t, s, gv, w, nv, vstride, err, skip, left, st);
     else
-      launch_nv<2, false>(P, t, s, gv, w, nv, vstride, err, skip, st);
+      launch_nv<2, false>(P, t, s, gv, w, nv, vstride, err, skip, left, st);
   } else {
     if (fp32)
-      launch_nv<3, true>(P, t, s, gv, w, nv, vstride, err, skip, st);
+      launch_nv<3, true>(P, t, s, gv, w, nv, vstride, err, skip, left, st);
     else
-      launch_nv<3, false>(P, t, s, gv, w, nv, vstride, err, skip, st);
+      launch_nv<3, false>(P, t, s, gv, w, nv, vstride, err, skip, left, st);
   }
 }
 

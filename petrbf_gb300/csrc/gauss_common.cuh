@@ -29,7 +29,7 @@ constexpr int kFxSymTile = 64;  // targets per pass of the fixed-point symmetric
 // ---- gauss_fx.cu: the FP64 sums with fixed-point exponents --------------------------------
 // Whether the plan's data fit it is plan.fx_ready (set with the point data).
 void gauss_fx_sum(const GaussPlan& P, const PointsView& t, const PointsView& s, const double* gv, double* w,
-                  unsigned* err, const int* skip, int nv, long long vstride, cudaStream_t st);
+                  unsigned* err, const int* skip, int nv, long long vstride, VecSkip left, cudaStream_t st);
 // The symmetric form's sum (2D, one vector; the partial slots are left for k_sym_gather).
 void gauss_fx_sym(const GaussPlan& P, const PointsView& s, const double* gv, double* w, unsigned* err,
                   const int* skip, cudaStream_t st);

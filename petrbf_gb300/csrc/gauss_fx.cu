@@ -146,13 +146,14 @@ struct FxArgs {
   double* part;
   long long pstride;
   int K, n, ncs;
+  VecSkip left;
 };
 
 // One pass of a consumer warp with N targets from t: buffers until the last one. Returns false
 // when a wait gave up.
 template <int DIM, int NV, bool SYM, int N>
-__device__ __forceinline__ bool fx_consume(unsigned char* smem, FxShared& sh, const FxArgs& a, int t, double norm,
-                                           int wid, int lane, int& b, unsigned& ph) {
+__device__ __forceinline__ bool fx_consume(unsigned char* smem, FxShared& sh, const FxArgs& a, const int (&vm)[NV],
+                                           int t, double norm, int wid, int lane, int& b, unsigned& ph) {
   using Lay = LayoutX<DIM, NV, SYM>;
   using C = CfgX<DIM, NV, SYM>;
   constexpr int KC = C::KC;
@@ -264,7 +265,7 @@ __device__ __forceinline__ bool fx_consume(unsigned char* smem, FxShared& sh, co
   }
   if (N > 0 && which >= 0) {
 #pragma unroll
-    for (int v = 0; v < NV; v++) a.w[v * a.vs + t + which] = run[v] * norm;
+    for (int v = 0; v < NV; v++) a.w[vm[v] * a.vs + t + which] = run[v] * norm;
   }
   return true;
 }
@@ -295,6 +296,8 @@ __global__ void __launch_bounds__(kFxThreads<SYM>, 2) k_gauss_fx(Grid g0, const 
                                                            const int* __restrict__ cs_s, FxArgs a, unsigned* err,
                                                            const int* __restrict__ skip) {
   if (skip && *skip) return;
+  int vm[NV];
+  if (!vec_map<NV>(a.left, vm)) return;
   using Lay = LayoutX<DIM, NV, SYM>;
   using C = CfgX<DIM, NV, SYM>;
   constexpr int NA = Lay::NA, RC = C::RC, KC = C::KC, TT = C::TT;
@@ -372,18 +375,18 @@ __global__ void __launch_bounds__(kFxThreads<SYM>, 2) k_gauss_fx(Grid g0, const 
         const int t = t0 + ta + u0;
         bool ok;
         switch (cnt) {
-          case 0: ok = fx_consume<DIM, NV, SYM, 0>(smem, sh, a, t, norm, wid, lane, b, ph); break;
-          case 1: ok = fx_consume<DIM, NV, SYM, 1>(smem, sh, a, t, norm, wid, lane, b, ph); break;
-          case 2: ok = fx_consume<DIM, NV, SYM, 2>(smem, sh, a, t, norm, wid, lane, b, ph); break;
-          case 3: ok = fx_consume<DIM, NV, SYM, 3>(smem, sh, a, t, norm, wid, lane, b, ph); break;
-          case 4: ok = fx_consume<DIM, NV, SYM, 4>(smem, sh, a, t, norm, wid, lane, b, ph); break;
+          case 0: ok = fx_consume<DIM, NV, SYM, 0>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+          case 1: ok = fx_consume<DIM, NV, SYM, 1>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+          case 2: ok = fx_consume<DIM, NV, SYM, 2>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+          case 3: ok = fx_consume<DIM, NV, SYM, 3>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+          case 4: ok = fx_consume<DIM, NV, SYM, 4>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
           default:
             if constexpr (C::TG == 8) {
               switch (cnt) {
-                case 5: ok = fx_consume<DIM, NV, SYM, 5>(smem, sh, a, t, norm, wid, lane, b, ph); break;
-                case 6: ok = fx_consume<DIM, NV, SYM, 6>(smem, sh, a, t, norm, wid, lane, b, ph); break;
-                case 7: ok = fx_consume<DIM, NV, SYM, 7>(smem, sh, a, t, norm, wid, lane, b, ph); break;
-                default: ok = fx_consume<DIM, NV, SYM, 8>(smem, sh, a, t, norm, wid, lane, b, ph); break;
+                case 5: ok = fx_consume<DIM, NV, SYM, 5>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+                case 6: ok = fx_consume<DIM, NV, SYM, 6>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+                case 7: ok = fx_consume<DIM, NV, SYM, 7>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+                default: ok = fx_consume<DIM, NV, SYM, 8>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
               }
             } else {
               ok = false;  // (not reached: at most TG targets a warp)
@@ -476,7 +479,7 @@ __global__ void __launch_bounds__(kFxThreads<SYM>, 2) k_gauss_fx(Grid g0, const 
           if (DIM == 3) bulk_g2s(dst + 2 * RC, a.sz + s_al, len * 8u, &sh.raw_bar[slot]);
 #pragma unroll
           for (int v = 0; v < NV; v++)
-            bulk_g2s(dst + (DIM + v) * RC, a.sg + v * a.vs + s_al, len * 8u, &sh.raw_bar[slot]);
+            bulk_g2s(dst + (DIM + v) * RC, a.sg + vm[v] * a.vs + s_al, len * 8u, &sh.raw_bar[slot]);
           bulk_g2s(dst + (DIM + NV) * RC, a.smask + s_al, len * 8u, &sh.raw_bar[slot]);
         }
       };
@@ -632,7 +635,7 @@ __global__ void __launch_bounds__(kFxThreads<SYM>, 2) k_gauss_fx(Grid g0, const 
 
 template <int DIM, int NV, bool BATCH, bool SYM>
 void launch_fx(const GaussPlan& P, const PointsView& t, const PointsView& s, const double* gv, double* w,
-               long long vstride, unsigned* err, const int* skip, cudaStream_t st) {
+               long long vstride, unsigned* err, const int* skip, VecSkip left, cudaStream_t st) {
   constexpr size_t sm = LayoutX<DIM, NV, SYM>::total;
   static_assert(sm <= 112 * 1024, "two CTAs of k_gauss_fx per SM");
   static std::atomic<bool> attr_set[64];  // per device: attribute set (idempotent, thread-safe)
@@ -645,7 +648,7 @@ void launch_fx(const GaussPlan& P, const PointsView& t, const PointsView& s, con
   }
   const DevBuf<uint2>* T = P.fx_self ? P.fxs : P.fxt;
   FxArgs a{T[0].get(), T[1].get(), T[2].get(), P.fxs[0].get(), P.fxs[1].get(), P.fxs[2].get(), P.smask.get(), gv,
-           vstride,    w,          nullptr,    0,              0,              s.n,            P.fx_ncs};
+           vstride,    w,          nullptr,    0,              0,              s.n,            P.fx_ncs, left};
   const int2* items = P.items.get();
   int nitems = P.nitems, grid = P.grid;
   if constexpr (SYM) {
@@ -670,40 +673,44 @@ void launch_fx(const GaussPlan& P, const PointsView& t, const PointsView& s, con
 
 template <int DIM>
 void sum_dim(const GaussPlan& P, const PointsView& t, const PointsView& s, const double* gv, double* w, int nv,
-             long long vs, unsigned* err, const int* skip, cudaStream_t st) {
+             long long vs, unsigned* err, const int* skip, VecSkip left, cudaStream_t st) {
   if (P.batched) {  // the problems are the segments of one vector
     for (int v = 0; v < nv; v++)
-      launch_fx<DIM, 1, true, false>(P, t, s, gv + v * vs, w + v * vs, vs, err, skip, st);
+      launch_fx<DIM, 1, true, false>(P, t, s, gv + v * vs, w + v * vs, vs, err, skip, VecSkip{}, st);
     return;
   }
   for (int v0 = 0; v0 < nv; v0 += 4) {
     const double* g0 = gv + v0 * vs;
     double* w0 = w + v0 * vs;
-    switch (std::min(4, nv - v0)) {
-      case 1: launch_fx<DIM, 1, false, false>(P, t, s, g0, w0, vs, err, skip, st); break;
-      case 2: launch_fx<DIM, 2, false, false>(P, t, s, g0, w0, vs, err, skip, st); break;
-      case 3: launch_fx<DIM, 3, false, false>(P, t, s, g0, w0, vs, err, skip, st); break;
-      default: launch_fx<DIM, 4, false, false>(P, t, s, g0, w0, vs, err, skip, st); break;
-    }
+    const int k0 = std::min(4, nv - v0);
+    const VecSkip l0 = vec_part(left, v0, k0);
+    for_counts(l0, k0, [&](int k) {
+      switch (k) {
+        case 1: launch_fx<DIM, 1, false, false>(P, t, s, g0, w0, vs, err, skip, l0, st); break;
+        case 2: launch_fx<DIM, 2, false, false>(P, t, s, g0, w0, vs, err, skip, l0, st); break;
+        case 3: launch_fx<DIM, 3, false, false>(P, t, s, g0, w0, vs, err, skip, l0, st); break;
+        default: launch_fx<DIM, 4, false, false>(P, t, s, g0, w0, vs, err, skip, l0, st); break;
+      }
+    });
   }
 }
 
 }  // namespace
 
 void gauss_fx_sum(const GaussPlan& P, const PointsView& t, const PointsView& s, const double* gv, double* w,
-                  unsigned* err, const int* skip, int nv, long long vstride, cudaStream_t st) {
+                  unsigned* err, const int* skip, int nv, long long vstride, VecSkip left, cudaStream_t st) {
   if (P.g.dim == 2)
-    sum_dim<2>(P, t, s, gv, w, nv, vstride, err, skip, st);
+    sum_dim<2>(P, t, s, gv, w, nv, vstride, err, skip, left, st);
   else
-    sum_dim<3>(P, t, s, gv, w, nv, vstride, err, skip, st);
+    sum_dim<3>(P, t, s, gv, w, nv, vstride, err, skip, left, st);
 }
 
 void gauss_fx_sym(const GaussPlan& P, const PointsView& s, const double* gv, double* w, unsigned* err,
                   const int* skip, cudaStream_t st) {
   if (P.batched)
-    launch_fx<2, 1, true, true>(P, s, s, gv, w, 0, err, skip, st);
+    launch_fx<2, 1, true, true>(P, s, s, gv, w, 0, err, skip, VecSkip{}, st);
   else
-    launch_fx<2, 1, false, true>(P, s, s, gv, w, 0, err, skip, st);
+    launch_fx<2, 1, false, true>(P, s, s, gv, w, 0, err, skip, VecSkip{}, st);
 }
 
 // The tables of gauss_fx.cuh, uploaded once per device.

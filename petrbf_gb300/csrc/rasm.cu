@@ -1318,8 +1318,11 @@ __global__ void __launch_bounds__(256, 2) k_apply_tri64(int ncell, const long lo
                                                      const double* __restrict__ Lpack, const double* __restrict__ r,
                                                      double* __restrict__ out, long long vs,
                                                      const int* __restrict__ skip, int full, double* __restrict__ Y,
-                                                     long long ys, SegSkip seg, const int* __restrict__ lu_of_cell) {
+                                                     long long ys, SegSkip seg, const int* __restrict__ lu_of_cell,
+                                                     VecSkip left) {
   if (skip && *skip) return;
+  int vm[NV];
+  if (!vec_map<NV>(left, vm)) return;
   if (seg.cell_done(blockIdx.x)) return;
   if (lu_of_cell && lu_of_cell[blockIdx.x] >= 0) return;  // factored by LU: k_apply_lu
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1338,7 +1341,7 @@ __global__ void __launch_bounds__(256, 2) k_apply_tri64(int ncell, const long lo
   for (int j = tid; j < nb; j += blockDim.x) {
     const int p = id[j < n1 ? nc + j : j - n1];
 #pragma unroll
-    for (int v = 0; v < NV; v++) y[v * nb + j] = r[v * vs + p];
+    for (int v = 0; v < NV; v++) y[v * nb + j] = r[vm[v] * vs + p];
   }
   // (warp 0) rows o .. o + np of the panel's triangle
   auto load_tri = [&](int o, int np) {
@@ -1492,11 +1495,11 @@ __global__ void __launch_bounds__(256, 2) k_apply_tri64(int ncell, const long lo
     double* Yc = Y + boff[c];
     for (int j = tid; j < nb; j += blockDim.x)
 #pragma unroll
-      for (int v = 0; v < NV; v++) Yc[v * ys + (j < n1 ? nc + j : j - n1)] = y[v * nb + j];
+      for (int v = 0; v < NV; v++) Yc[vm[v] * ys + (j < n1 ? nc + j : j - n1)] = y[v * nb + j];
   } else {
     for (int i = tid; i < nc; i += blockDim.x)
 #pragma unroll
-      for (int v = 0; v < NV; v++) out[v * vs + cs[c] + i] = y[v * nb + n1 + i];
+      for (int v = 0; v < NV; v++) out[vm[v] * vs + cs[c] + i] = y[v * nb + n1 + i];
   }
 }
 
@@ -1523,8 +1526,10 @@ __global__ void __launch_bounds__(kTrwWarps * 32) k_apply_trw(int ncell, const l
                                                              const double* __restrict__ r, double* __restrict__ out,
                                                              long long vs, const int* __restrict__ skip, int full,
                                                              double* __restrict__ Y, long long ys, SegSkip seg,
-                                                             int ldy) {
+                                                             int ldy, VecSkip left) {
   if (skip && *skip) return;
+  int vm[NV];
+  if (!vec_map<NV>(left, vm)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int c = blockIdx.x * kTrwWarps + wid;
@@ -1539,7 +1544,7 @@ __global__ void __launch_bounds__(kTrwWarps * 32) k_apply_trw(int ncell, const l
   for (int j = lane; j < nb; j += 32) {
     const int p = id[j < n1 ? nc + j : j - n1];
 #pragma unroll
-    for (int v = 0; v < NV; v++) y[v * ldy + j] = (float)r[v * vs + p];
+    for (int v = 0; v < NV; v++) y[v * ldy + j] = (float)r[vm[v] * vs + p];
   }
   __syncwarp();
   // ---- forward: L y = r ----
@@ -1848,10 +1853,11 @@ __global__ void __launch_bounds__(kLuThreads) k_apply_lu(int nlu, const int* __r
 // basic Schwarz: out[i] = sum of the slots of point i (ascending slot = ascending block)
 __global__ void k_asm_gather(int n, int nv, const long long* __restrict__ inv_off,
                              const long long* __restrict__ inv_slot, const double* __restrict__ Y, long long ys,
-                             double* __restrict__ out, long long vs, const int* __restrict__ skip) {
+                             double* __restrict__ out, long long vs, const int* __restrict__ skip, VecSkip left) {
   if (skip && *skip) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     for (int v = 0; v < nv; v++) {
+      if (left.done && left.done[(long long)v * left.stride]) continue;
       double s = 0.0;
       for (long long k = inv_off[i]; k < inv_off[i + 1]; k++) s += Y[v * ys + inv_slot[k]];
       out[v * vs + i] = s;
@@ -2226,38 +2232,26 @@ int trw_ldy(const RasmPlan& R) { return (std::max(R.max_nb, 1) + 3) & ~3; }
 
 template <class T>
 void apply_tri_nv(const RasmPlan& R, const T* Lp, const int* cs, const double* r, double* out, long long vs, int nv,
-                  cudaStream_t s, const int* skip) {
+                  cudaStream_t s, const int* skip, VecSkip left) {
   const int full = R.basic ? 1 : 0;
-  if constexpr (std::is_same<T, float>::value) {
-    const int ldy = trw_ldy(R);
-    const size_t sm = (size_t)kTrwWarps * nv * ldy * sizeof(float);
-    const int grid = ceil_div(R.ncell, kTrwWarps);
-    switch (nv) {
-      case 1:
-        k_apply_trw<1><<<grid, kTrwWarps * 32, sm, s>>>(R.ncell, R.boff.get(), cs, R.idx.get(), R.loff.get(), Lp, r,
-                                                        out, vs, skip, full, R.Y.get(), R.nslot, R.seg, ldy);
-        break;
-      case 2:
-        k_apply_trw<2><<<grid, kTrwWarps * 32, sm, s>>>(R.ncell, R.boff.get(), cs, R.idx.get(), R.loff.get(), Lp, r,
-                                                        out, vs, skip, full, R.Y.get(), R.nslot, R.seg, ldy);
-        break;
-      case 3:
-        k_apply_trw<3><<<grid, kTrwWarps * 32, sm, s>>>(R.ncell, R.boff.get(), cs, R.idx.get(), R.loff.get(), Lp, r,
-                                                        out, vs, skip, full, R.Y.get(), R.nslot, R.seg, ldy);
-        break;
-      default:
-        k_apply_trw<4><<<grid, kTrwWarps * 32, sm, s>>>(R.ncell, R.boff.get(), cs, R.idx.get(), R.loff.get(), Lp, r,
-                                                        out, vs, skip, full, R.Y.get(), R.nslot, R.seg, ldy);
-        break;
+  for_counts(left, nv, [&](int k) {
+    if constexpr (std::is_same<T, float>::value) {
+      const int ldy = trw_ldy(R);
+      const size_t sm = (size_t)kTrwWarps * k * ldy * sizeof(float);
+      const auto f = k == 1 ? k_apply_trw<1> : k == 2 ? k_apply_trw<2> : k == 3 ? k_apply_trw<3> : k_apply_trw<4>;
+      f<<<ceil_div(R.ncell, kTrwWarps), kTrwWarps * 32, sm, s>>>(R.ncell, R.boff.get(), cs, R.idx.get(), R.loff.get(),
+                                                                 Lp, r, out, vs, skip, full, R.Y.get(), R.nslot, R.seg,
+                                                                 ldy, left);
+    } else {
+      const size_t sm = (size_t)k * R.max_nb * sizeof(double);
+      const int* luc = R.nlu ? R.lu_of_cell.get() : nullptr;
+      const auto f =
+          k == 1 ? k_apply_tri64<1> : k == 2 ? k_apply_tri64<2> : k == 3 ? k_apply_tri64<3> : k_apply_tri64<4>;
+      f<<<R.ncell, tri64_threads(R), sm, s>>>(R.ncell, R.boff.get(), cs, R.idx.get(), R.loff.get(), Lp, r, out, vs,
+                                              skip, full, R.Y.get(), R.nslot, R.seg, luc, left);
     }
-  } else {
-    const size_t sm = (size_t)nv * R.max_nb * sizeof(double);
-    const int* luc = R.nlu ? R.lu_of_cell.get() : nullptr;
-    const auto k = nv == 1 ? k_apply_tri64<1> : nv == 2 ? k_apply_tri64<2> : nv == 3 ? k_apply_tri64<3> : k_apply_tri64<4>;
-    k<<<R.ncell, tri64_threads(R), sm, s>>>(R.ncell, R.boff.get(), cs, R.idx.get(), R.loff.get(), Lp, r, out, vs, skip,
-                                            full, R.Y.get(), R.nslot, R.seg, luc);
-  }
-  PRBF_CHECK_LAUNCH();
+    PRBF_CHECK_LAUNCH();
+  });
 }
 
 template <class T>
@@ -2283,18 +2277,19 @@ void set_tri_smem(const RasmPlan& R) {
 }  // namespace
 
 void rasm_apply(const RasmPlan& R, const int* cs, const double* r, double* out, cudaStream_t s, const int* skip, int nv,
-                long long vstride) {
+                long long vstride, VecSkip left) {
   if (R.nblocks == 0 || nv <= 0) return;
   const int step = std::max(1, std::min(4, R.max_nv));
   for (int v0 = 0; v0 < nv; v0 += step) {
     const int k = std::min(step, nv - v0);
     const double* rv = r + v0 * vstride;
     double* ov = out + v0 * vstride;
+    const VecSkip lv = vec_part(left, v0, k);
     if (R.factor) {
       if (R.fp32) {
-        apply_tri_nv<float>(R, R.L32.get(), cs, rv, ov, vstride, k, s, skip);
+        apply_tri_nv<float>(R, R.L32.get(), cs, rv, ov, vstride, k, s, skip, lv);
       } else {
-        apply_tri_nv<double>(R, R.L64.get(), cs, rv, ov, vstride, k, s, skip);
+        apply_tri_nv<double>(R, R.L64.get(), cs, rv, ov, vstride, k, s, skip, lv);
         if (R.nlu) {
           k_apply_lu<<<R.nlu, kLuThreads, (size_t)k * R.max_nb * sizeof(double), s>>>(
               R.nlu, R.lucell.get(), R.boff.get(), cs, R.idx.get(), R.lukoff.get(), R.LU64.get(), R.lupoff.get(),
@@ -2313,7 +2308,7 @@ void rasm_apply(const RasmPlan& R, const int* cs, const double* r, double* out, 
     }
     if (R.basic) {
       k_asm_gather<<<ceil_div(R.n, 256), 256, 0, s>>>(R.n, k, R.inv_off.get(), R.inv_slot.get(), R.Y.get(), R.nslot,
-                                                      ov, vstride, skip);
+                                                      ov, vstride, skip, lv);
       PRBF_CHECK_LAUNCH();
     }
   }

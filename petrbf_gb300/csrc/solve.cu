@@ -37,11 +37,25 @@ struct GaussRasmOp : Operator {
   unsigned* err = nullptr;
   int nv = 1;
   long long vstride = 0;
+  // the Krylov iterations (skip given) leave out the right-hand sides that have stopped: a
+  // vortex ring's third component is zero and stops at once. Each operation is then launched
+  // once per count that may be left, about 2 us for those that return: from kLeaveOut points
+  const KSeg* seg = nullptr;
+  static constexpr int kLeaveOut = 4096;
+  VecSkip left(const int* skip) const {
+    VecSkip k;
+    if (skip && seg && nv > 1 && v.n >= kLeaveOut) {
+      k.done = &seg->done;
+      k.stride = (int)(sizeof(KSeg) / sizeof(int));
+      k.nv = nv;
+    }
+    return k;
+  }
   void apply_A(const double* x, double* y, const int* skip, cudaStream_t s) const override {
-    gauss_sum_dev(*plan, v, v, x, y, fp32, err, s, skip, nv, vstride);
+    gauss_sum_dev(*plan, v, v, x, y, fp32, err, s, skip, nv, vstride, left(skip));
   }
   void apply_B(const double* r, double* z, const int* skip, cudaStream_t s) const override {
-    rasm_apply(*rasm, v.cell_start, r, z, s, skip, nv, vstride);
+    rasm_apply(*rasm, v.cell_start, r, z, s, skip, nv, vstride, left(skip));
   }
 };
 
@@ -144,6 +158,7 @@ static void interpolate(Ctx& c, int n, const double* x, const double* y, const d
   for (int v = 0; v < nv; v++) offs[v] = v * ldn;
   if (!S.kry.same_layout(offs, lens, p.restart)) S.kry.init(offs, lens, len_all, p.restart, c.stream);
   S.kry.graph_op = nullptr;  // operators are rebuilt per call
+  S.op64.seg = S.op32.seg = S.kry.st.get();
 
   const bool use_guess = p.guess == PRBF_GUESS_LEARNED;
   if (use_guess && (dim != 2 || !c.guess || !c.guess->ready))
@@ -221,7 +236,13 @@ static void interpolate(Ctx& c, int n, const double* x, const double* y, const d
       if (xzero) {
         PRBF_CUDA(cudaMemcpyAsync(S.r.get(), S.b.get(), sizeof(double) * nall, cudaMemcpyDeviceToDevice, c.stream));
       } else {
+        // (the right-hand sides up to the last that has not stopped; not fewer than two of
+        // several, whose sums round alike whatever their number)
+        S.op64.nv = std::min(nv, 2);
+        for (int v = 0; v < nv; v++)
+          if (!reason[v]) S.op64.nv = std::max(S.op64.nv, v + 1);
         S.op64.apply_A(S.x.get(), S.tmp.get(), nullptr, c.stream);
+        S.op64.nv = nv;
         PRBF_CUDA(cudaMemcpyAsync(S.r.get(), S.b.get(), sizeof(double) * nall, cudaMemcpyDeviceToDevice, c.stream));
         axpy_dev(nall, -1.0, S.tmp.get(), S.r.get(), c.stream);
       }

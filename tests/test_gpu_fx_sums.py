@@ -112,3 +112,28 @@ def test_several_vectors(dim, nrhs):
     for k in range(nrhs):
         r = O.matvec(gr, p[0][perm], p[1][perm], pz, cs, g[perm, k]) - f[perm, k]
         assert np.linalg.norm(r) <= 1e-10 * np.linalg.norm(f[:, k])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("stopped", [0, 1, 2])
+def test_stopped_right_hand_sides_are_left_out(precision, stopped):
+    # a zero right-hand side among three stops at once, the others go on without it (from 4096
+    # points); weights against the oracle's residual, as above
+    m = 18
+    h = 2.0 / m
+    rng = np.random.default_rng(stopped)
+    ax = np.meshgrid(*([-1 + h * np.arange(m)] * 3), indexing="ij")
+    x, y, z = (a.ravel() + rng.uniform(-0.2 * h, 0.2 * h, a.size) for a in ax)
+    prm = (h, 3, 7, 17)
+    f = np.stack([np.cos((k + 1) * x) * y for k in range(3)], axis=1)
+    f[:, stopped] = 0.0
+    with Context(dim=3, sigma=prm[0], nsigma_box=prm[1], sigma_buffer=prm[2], sigma_trunc=prm[3], pc="asm",
+                 precision=precision) as c:
+        g, _ = c.interpolate(x, y, z, f)
+    assert not g[:, stopped].any()
+    gr = O.grid_for(x, y, z, *prm)
+    perm, cs = O.cell_sort(gr, x, y, z)
+    for k in range(3):
+        if k != stopped:
+            r = O.matvec(gr, x[perm], y[perm], z[perm], cs, g[perm, k]) - f[perm, k]
+            assert np.linalg.norm(r) <= 1e-10 * np.linalg.norm(f[:, k])
