@@ -132,6 +132,11 @@ __global__ void k_split_hl(long long n, const double* __restrict__ v, float2* __
 // FP32 rows of the block assembly: one warp, lanes along row i (columns 0..i), the split
 // coordinates from shared memory, the exponential as the FP32 sums take it (ex2.approx);
 // the diagonal shift is added by the lane that wrote the diagonal.
+// FP32 blocks as the tensor-core factorisation reads them (k_chol_tc).
+// Row pitch (floats) of a block of nbp rows in memory: whole 128-byte lines.
+__host__ __device__ __forceinline__ int tc_pitch(int nbp) { return (nbp + 31) & ~31; }
+// S_c form: empty rows and columns between the neighbours (n1) and the centre points.
+__host__ __device__ __forceinline__ int tc_pad(int n1) { return -n1 & 3; }
 __device__ __forceinline__ float asm_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -139,7 +144,7 @@ __device__ __forceinline__ float asm_ex2(float x) {
 }
 template <int DIM>
 __device__ __forceinline__ void asm_row_f32(float* __restrict__ Arow, const float2* s_hl, int nbk, int i, float c2,
-                                            float sh, int lane) {
+                                            float sh, int lane, int nl, int pad) {
   float2 ha[DIM];
 #pragma unroll
   for (int d = 0; d < DIM; d++) ha[d] = s_hl[d * nbk + i];
@@ -151,9 +156,9 @@ __device__ __forceinline__ void asm_row_f32(float* __restrict__ Arow, const floa
       const float dd = (ha[d].x - hb.x) + (ha[d].y - hb.y);
       r2 = fmaf(dd, dd, r2);
     }
-    Arow[j] = asm_ex2(-r2 * c2);
+    Arow[j < nl ? j : j + pad] = asm_ex2(-r2 * c2);
   }
-  if (sh != 0.f && lane == (i & 31)) Arow[i] += sh;
+  if (sh != 0.f && lane == (i & 31)) Arow[i < nl ? i : i + pad] += sh;
 }
 
 template <class T>
@@ -163,7 +168,7 @@ __global__ void k_assemble(int nblk, const int* __restrict__ blk_cell, const lon
                            const double* __restrict__ y, const double* __restrict__ z, int dim, double inv2s2_all,
                            const double* __restrict__ cell_sig, double shift, T* __restrict__ K,
                            const unsigned char* __restrict__ only, const float2* __restrict__ hl, long long n,
-                           double kexp_all, const double* __restrict__ tab) {
+                           double kexp_all, const double* __restrict__ tab, int restricted) {
   int b = blockIdx.y;
   if (b >= nblk || (only && !only[b])) return;
   int c = blk_cell[b];
@@ -187,13 +192,20 @@ __global__ void k_assemble(int nblk, const int* __restrict__ blk_cell, const lon
   // a warp per row (rows dealt round-robin over the block's CTAs and warps), lanes along it
   const int nw = blockDim.x >> 5, lane = threadIdx.x & 31;
   if constexpr (std::is_same<T, float>::value) {
+    // rows at the tensor-core factorisation's pitch, its empty rows and columns zero
     const float c2 = (float)(inv2s2 * 1.4426950408889634), sh = (float)shift;
+    const int pad = restricted ? tc_pad(n1) : 0, ld = tc_pitch(nbk + pad);
+    const int nl = restricted ? n1 : nbk;  // columns from nl on move by pad
     for (int i = blockIdx.x * nw + (threadIdx.x >> 5); i < nbk; i += gridDim.x * nw) {
+      float* Arow = A + (long long)(i < nl ? i : i + pad) * ld;
       if (dim == 3)
-        asm_row_f32<3>(A + (long long)i * nbk, s_hl, nbk, i, c2, sh, lane);
+        asm_row_f32<3>(Arow, s_hl, nbk, i, c2, sh, lane, nl, pad);
       else
-        asm_row_f32<2>(A + (long long)i * nbk, s_hl, nbk, i, c2, sh, lane);
+        asm_row_f32<2>(Arow, s_hl, nbk, i, c2, sh, lane, nl, pad);
+      if (i >= nl && lane < pad) Arow[nl + lane] = 0.f;
     }
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < pad * (nl + pad); e += gridDim.x * blockDim.x)
+      A[(long long)(nl + e / (nl + pad)) * ld + e % (nl + pad)] = 0.f;
   } else {
     for (int i = blockIdx.x * nw + (threadIdx.x >> 5); i < nbk; i += gridDim.x * nw) {
       const int pa = id[i < n1 ? nc + i : i - n1];
@@ -656,22 +668,35 @@ __device__ bool potrf_trtri_w(float* C, float* M, int h) {
 // accuracy comes from splitting every operand x = hi + lo (hi = x rounded to TF32, lo =
 // the rest, also TF32): A B ~ Ahi Bhi + Ahi Blo + Alo Bhi. Operands go through shared
 // memory in 32-column chunks in the canonical K-major layout without swizzle (core
-// matrices of 8 rows x 16 bytes; element (r, k) at (r/8)*SBO + (k/4)*128 + (r%8)*16 +
-// (k%4)*4 bytes, SBO = 8 core matrices = 1024 bytes, LBO = 128 bytes). One elected thread
-// issues the MMAs and commits them to an mbarrier; the diagonal tiles are factored and
-// inverted on the CUDA cores (potrf_trtri_w). Writes L (lower part) over the dense block;
-// the factor form then packs it (k_pack_factor), the restricted S_c form computes S_c in
-// the same kernel from L and the diagonal inverses (below).
+// matrices of 8 rows x 16 bytes; element (r, k) at (r/8)*SBO + (k/4)*LBO + (r%8)*16 +
+// (k%4)*4 bytes). A thread moves 16-byte units of a row, the eight lanes of a quarter warp
+// one row's 128 bytes, so the global loads are whole lines; LBO = 144 bytes (a core matrix
+// and 16 bytes) puts the eight units of such a row into eight different bank groups, so the
+// stores are free of conflicts too. That needs rows of K at 16-byte boundaries: a block is
+// held with a row pitch of tc_pitch() floats, and in the S_c form its centre rows and
+// columns start at the next multiple of four (tc_pad(); the rows and columns between hold
+// zeros). One elected thread issues the MMAs and commits them to an mbarrier; the diagonal
+// tiles are factored and inverted on the CUDA cores (potrf_trtri_w). The updated panel goes
+// from the update's epilogue straight into the panel solve's operand (registers). Three CTAs
+// per SM (72 KB and 80 registers) cover one another's waits. Writes L (lower part) over the
+// dense block; the factor form then packs it (k_pack_factor), the restricted S_c form
+// computes S_c in the same kernel from L and the diagonal inverses (below).
+// Bound by the latency of the chain from chunk to chunk (loads, split, barrier, MMAs) and of
+// the pivots; tensor pipe 20 % busy, L1 49 %. With 4-byte accesses of the units (eight lines a
+// load instruction) and two CTAs per SM, the L1's line lookups set the time: 1600 blocks of 870
+// points, S_c form, 17.4 -> 9.9 ms. Asking the L2 for chunks ahead of their loads gains nothing.
 constexpr int TC_KCH = 32;  // K columns per operand chunk
 
 __device__ __forceinline__ uint32_t tc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 
+constexpr int TC_LBO = 144, TC_SBO = (TC_KCH / 4) * TC_LBO;  // bytes
+constexpr int TC_A = 128 / 8 * TC_SBO / 4, TC_B = 64 / 8 * TC_SBO / 4;  // floats of an operand
+
 __device__ __forceinline__ uint64_t tc_desc(uint32_t addr) {
-  constexpr uint32_t lbo = 128, sbo = (TC_KCH / 4) * 128;
   uint64_t d = (uint64_t)((addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)(lbo >> 4) << 16;
-  d |= (uint64_t)(sbo >> 4) << 32;
+  d |= (uint64_t)(TC_LBO >> 4) << 16;
+  d |= (uint64_t)(TC_SBO >> 4) << 32;
   d |= (uint64_t)1 << 46;  // descriptor version for tcgen05; base offset 0, no swizzle
   return d;
 }
@@ -682,9 +707,9 @@ __device__ __forceinline__ void tc_split(float x, float& hi, float& lo) {
 }
 
 struct TcStage {
-  float* ahi;  // [128][TC_KCH] canonical
+  float* ahi;  // 128 rows
   float* alo;
-  float* bhi;  // [64][TC_KCH]
+  float* bhi;  // 64 rows
   float* blo;
 };
 
@@ -698,7 +723,7 @@ __device__ __forceinline__ void tc_issue(uint32_t tmem, const TcStage& st, bool 
   for (int ks = 0; ks < TC_KCH / 8; ks++)
 #pragma unroll
     for (int t = 0; t < 3; t++) {
-      const uint64_t da = tc_desc(tc_smem(as[t]) + ks * 256), db = tc_desc(tc_smem(bs[t]) + ks * 256);
+      const uint64_t da = tc_desc(tc_smem(as[t]) + ks * 2 * TC_LBO), db = tc_desc(tc_smem(bs[t]) + ks * 2 * TC_LBO);
       const uint32_t acc = (first && ks == 0 && t == 0) ? 0u : 1u;
       asm volatile(
           "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}" ::"r"(
@@ -725,147 +750,219 @@ __device__ __forceinline__ void tc_sync() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-// 32 columns of the thread's TMEM row: warp w reads lanes 32 (w % 4) .., column half w / 4
-__device__ __forceinline__ void tc_load32(uint32_t tmem, float v[32]) {
-  const int w = threadIdx.x >> 5;
-  const uint32_t addr = tmem + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)(32 * (w >> 2));
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
-      "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(addr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int j = 0; j < 32; j++) v[j] = __uint_as_float(r[j]);
-}
-
-// One operand chunk in registers: A rows [ar0, ar0 + 128) (valid below ar_end and at or
-// above ar_skip), columns [c0, c0 + 32) (valid below c_end) of the dense block, and B rows
-// [br0, br0 + 64) (valid below br_end) from the dense block (Msm null) or from the diagonal
-// inverse M in shared memory. Each warp instruction covers one core matrix (8 rows x 4
-// columns: lane l -> row l/4, column l%4), so the global loads touch 8 row segments of 16
-// bytes and the shared-memory stores are 32 consecutive words; all loads are issued before
-// any is used.
-struct TcRegs {
-  float a[16], b[8];
+// One CTA's tensor-core state and the units its threads move: unit (r, kg) is 16 bytes of row
+// r, columns 4 kg .. 4 kg + 3 of a chunk, at rows tr + 32 i of an operand for each thread.
+struct Tc {
+  TcStage st;
+  float* Et;  // [128][S] result staging, over the idle operand stage
+  float* Ct;  // [TB][S] diagonal tile, over the stage behind Et
+  float* Mt;  // [TB][S] inverse of the diagonal tile
+  uint64_t* bar;
+  int* s_abort;
+  unsigned* err;
+  uint32_t tmem;
+  unsigned phase;
 };
+constexpr int kTcS = SP<float>::S;
+constexpr int kTcStage = 2 * TC_A + 2 * TC_B;  // floats
+static_assert((128 + TB) * kTcS <= kTcStage, "the result and diagonal tiles fit the operand stage");
+static_assert(NTH == 256 && TB == 64 && TC_KCH == 32, "the thread to unit maps below");
 
-// Bsrc: the matrix the B rows come from when not from Msm (same row stride nb as A); bt:
-// B is the transpose of Bsrc, element (r, k) at Bsrc[(c0 + k) nb + br0 + r] (a warp
-// instruction then reads 4 rows of Bsrc, 32 contiguous bytes each).
-__device__ __forceinline__ void tc_fetch(TcRegs& R, const float* A, int nb, int ar0, int ar_skip, int ar_end, int c0,
-                                         int c_end, int br0, int br_end, const float* Msm, int mcol0,
-                                         const float* Bsrc = nullptr, bool bt = false) {
-  constexpr int S = SP<float>::S;
-  if (!Bsrc) Bsrc = A;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+size_t chol_tc_smem() { return sizeof(float) * (kTcStage + TB * kTcS) + 64; }
+
+__device__ __forceinline__ int tc_tr() { return 4 * (threadIdx.x >> 5) + ((threadIdx.x & 31) >> 3); }
+__device__ __forceinline__ int tc_kg() { return threadIdx.x & 7; }
+
+// bit i: row row0 + tr + 32 i lies in [lo, hi)
+__device__ __forceinline__ unsigned tc_rows(int row0, int lo, int hi) {
+  unsigned m = 0;
 #pragma unroll
-  for (int i = 0; i < 16; i++) {  // A: core matrices w*16 + i (row group cm/8, column group cm%8)
-    const int cm = w * 16 + i, r = (cm >> 3) * 8 + (lane >> 2), k = (cm & 7) * 4 + (lane & 3);
-    const int row = ar0 + r;
-    R.a[i] = (row < ar_end && row >= ar_skip && c0 + k < c_end) ? A[(long long)row * nb + c0 + k] : 0.f;
+  for (int i = 0; i < 4; i++) {
+    const int row = row0 + tc_tr() + 32 * i;
+    m |= (row >= lo && row < hi ? 1u : 0u) << i;
   }
-#pragma unroll
-  for (int i = 0; i < 8; i++) {  // B: core matrices w*8 + i
-    const int cm = w * 8 + i, r = (cm >> 3) * 8 + (lane >> 2), k = (cm & 7) * 4 + (lane & 3);
-    const int row = br0 + r;
-    float x = 0.f;
-    if (row < br_end) {
-      if (Msm)
-        x = Msm[r * S + mcol0 + k];
-      else if (c0 + k < c_end)
-        x = bt ? Bsrc[(long long)(c0 + k) * nb + row] : Bsrc[(long long)row * nb + c0 + k];
+  return m;
+}
+
+// Unit i of the thread into an operand's hi and lo parts (o: word offset of its first unit).
+__device__ __forceinline__ void tc_put(float* hi, float* lo, int o, float4 v) {
+  float4 h, l;
+  tc_split(v.x, h.x, l.x);
+  tc_split(v.y, h.y, l.y);
+  tc_split(v.z, h.z, l.z);
+  tc_split(v.w, h.w, l.w);
+  *(float4*)(hi + o) = h;
+  *(float4*)(lo + o) = l;
+}
+__device__ __forceinline__ int tc_off(int r, int kg) { return ((r >> 3) * TC_SBO + kg * TC_LBO + (r & 7) * 16) / 4; }
+
+// Issue the staged chunk's MMAs and wait for them; false (error flagged) if the commit is not
+// seen in time. `between` runs while the tensor cores work.
+template <class F>
+__device__ __forceinline__ bool tc_chunk(Tc& T, bool first, F between) {
+  tc_sync();
+  if (threadIdx.x == 0) tc_issue(T.tmem, T.st, first);
+  between();
+  if (!tc_commit_wait(T.bar, T.phase)) {
+    if (threadIdx.x == 0) {
+      atomicOr(T.err, DEV_ERR_TIMEOUT);
+      *T.s_abort = 1;
     }
-    R.b[i] = x;
   }
+  __syncthreads();
+  return *T.s_abort == 0;
 }
 
-// Core matrix cm of a chunk occupies words [32 cm, 32 cm + 32) in the canonical layout.
-__device__ __forceinline__ void tc_store(const TcStage& st, const TcRegs& R) {
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// D (TMEM, 128 x 64) = sum over the columns [k0, k1) of the rows [ar0, ar0 + 128) (below
+// ar_end) of Asrc times B^T: B the rows [br0, br0 + bh) of Bsrc or, with BT, of its transpose
+// (element (r, k) at Bsrc[k ld + br0 + r]; a warp reads 32 consecutive floats of a row). k0 and
+// the rows' starts are multiples of four floats. The next chunk's loads are in flight while the
+// tensor cores work. A unit that reaches past k1 reads zeros there: the empty columns, or rows
+// that BT leaves out.
+template <bool BT>
+__device__ __forceinline__ bool tc_sum(Tc& T, const float* Asrc, int ld, int ar0, int ar_end, const float* Bsrc,
+                                       int br0, int bh, int k0, int k1) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, tr = tc_tr(), kg = tc_kg();
+  const unsigned am = tc_rows(ar0, 0, ar_end), bm = tc_rows(0, 0, bh);
+  const float* pa = Asrc + (long long)(ar0 + tr) * ld + 4 * kg;
+  const int br = BT ? (w & 1) * 32 + lane : tr, bk = BT ? w >> 1 : kg;
+  const float* pb = BT ? Bsrc + (long long)(4 * bk) * ld + br0 + br : Bsrc + (long long)(br0 + tr) * ld + 4 * kg;
+  float4 a[4], b[2];
+  auto fetch = [&](int c0) {
+    const bool in = c0 + 4 * kg < k1;
 #pragma unroll
-  for (int i = 0; i < 16; i++) {
-    float h, l;
-    tc_split(R.a[i], h, l);
-    st.ahi[(w * 16 + i) * 32 + lane] = h;
-    st.alo[(w * 16 + i) * 32 + lane] = l;
-  }
+    for (int i = 0; i < 4; i++)
+      a[i] = in && (am >> i & 1) ? *(const float4*)(pa + (long long)(32 * i) * ld + c0) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
-    float h, l;
-    tc_split(R.b[i], h, l);
-    st.bhi[(w * 8 + i) * 32 + lane] = h;
-    st.blo[(w * 8 + i) * 32 + lane] = l;
-  }
-}
-
-size_t chol_tc_smem() {
-  return sizeof(float) * (2 * 128 * TC_KCH + 2 * 64 * TC_KCH + 2 * TB * SP<float>::S) + 64;
-}
-
-// The MMA pipeline of one 128 x 64 product: D (TMEM) = sum over the columns [k0, k1) of
-// Asrc rows [ar0, ar0 + 128) (valid in [ar_skip, ar_end)) times B^T, B the rows [br0,
-// br_end) of Bsrc (of its transpose with bt) or, with Msm, the rows of M in shared memory at
-// column c - k0. Chunks of 32 columns; the next chunk's loads are in flight while the tensor
-// cores work. Returns false (error flagged, s_abort set) if an MMA commit is not seen in time.
-__device__ bool tc_gemm(const TcStage& st, uint32_t tmem, uint64_t* bar, unsigned& phase, int* s_abort,
-                        unsigned* err, const float* Asrc, int ld, int ar0, int ar_skip, int ar_end, const float* Bsrc,
-                        int br0, int br_end, const float* Msm, int k0, int k1, bool bt = false) {
-  TcRegs R;
-  tc_fetch(R, Asrc, ld, ar0, ar_skip, ar_end, k0, k1, br0, br_end, Msm, 0, Bsrc, bt);
-  for (int c0 = k0; c0 < k1; c0 += TC_KCH) {
-    tc_store(st, R);
-    tc_sync();
-    if (threadIdx.x == 0) tc_issue(tmem, st, c0 == k0);
-    if (c0 + TC_KCH < k1)
-      tc_fetch(R, Asrc, ld, ar0, ar_skip, ar_end, c0 + TC_KCH, k1, br0, br_end, Msm, c0 + TC_KCH - k0, Bsrc, bt);
-    if (!tc_commit_wait(bar, phase)) {
-      if (threadIdx.x == 0) {
-        atomicOr(err, DEV_ERR_TIMEOUT);
-        *s_abort = 1;
+    for (int i = 0; i < 2; i++) {
+      if constexpr (BT) {
+        float* v = (float*)&b[i];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const int c = c0 + 16 * i + j;
+          v[j] = br < bh && c + 4 * bk < k1 ? pb[(long long)c * ld] : 0.f;
+        }
+      } else {
+        b[i] = in && (bm >> i & 1) ? *(const float4*)(pb + (long long)(32 * i) * ld + c0) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
-    __syncthreads();
-    if (*s_abort) return false;
+  };
+  fetch(k0);
+  for (int c0 = k0; c0 < k1; c0 += TC_KCH) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) tc_put(T.st.ahi, T.st.alo, tc_off(tr + 32 * i, kg), a[i]);
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+      tc_put(T.st.bhi, T.st.blo, BT ? tc_off(br, bk + 4 * i) : tc_off(tr + 32 * i, kg), b[i]);
+    if (!tc_chunk(T, c0 == k0, [&] {
+          if (c0 + TC_KCH < k1) fetch(c0 + TC_KCH);
+        }))
+      return false;
   }
   return true;
 }
 
-// The 128 x 64 result in TMEM through shared memory (Et, over the idle operand stage) into
-// dst rows [r0, r0 + 128) below r_end, columns [c0, c0 + h): dst -= D (sub) or dst = D.
-__device__ void tc_epi(uint32_t tmem, float* Et, float* dst, long long ld, int r0, int r_end, int c0, int h, bool sub) {
-  constexpr int kEtS = TB + 1;
-  const int tid = threadIdx.x, w = tid >> 5;
-  {
-    float v[32];
-    tc_load32(tmem, v);
-    const int r_own = 32 * (w & 3) + (tid & 31), cbase = 32 * (w >> 2);
+// The 128 x 64 result in TMEM to Et: warp w reads TMEM lanes 32 (w % 4) .., column half w / 4.
+__device__ __forceinline__ void tc_drain(const Tc& T) {
+  const int w = threadIdx.x >> 5, row = 32 * (w & 3) + (threadIdx.x & 31);
 #pragma unroll
-    for (int j = 0; j < 32; j++) Et[r_own * kEtS + cbase + j] = v[j];
-  }
-  __syncthreads();
-  constexpr int kRmw = 8;
-  for (int e0 = 0; e0 < 128 * TB; e0 += kRmw * NTH) {
-    float a[kRmw];
+  for (int half = 0; half < 2; half++) {
+    const int col = 32 * (w >> 2) + 16 * half;
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(T.tmem + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)col));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int g = 0; g < kRmw; g++) {
-      const int e = e0 + g * NTH + tid, rr = e / TB, col = e % TB, row = r0 + rr;
-      a[g] = (sub && row < r_end && col < h) ? dst[(long long)row * ld + c0 + col] : 0.f;
-    }
-#pragma unroll
-    for (int g = 0; g < kRmw; g++) {
-      const int e = e0 + g * NTH + tid, rr = e / TB, col = e % TB, row = r0 + rr;
-      if (row < r_end && col < h) dst[(long long)row * ld + c0 + col] = sub ? a[g] - Et[rr * kEtS + col] : Et[rr * kEtS + col];
-    }
+    for (int j = 0; j < 16; j++) T.Et[row * kTcS + col + j] = __uint_as_float(r[j]);
   }
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(NTH, 2) k_chol_tc(int nblk, const int* __restrict__ blk_cell,
+// A panel's values in the units of the panel solve's operand: V[half][i] holds row tr + 32 i,
+// columns 32 half + 4 kg ...
+struct TcPanel {
+  float4 v[2][4];
+};
+
+// V = C - D, C the rows [row0, row0 + 128) (those in rm) of src at columns c0 .. c0 + h, or
+// (src null) the identity's at column offset ident (< 0 none: zero); D the sum in TMEM (have)
+// or zero.
+__device__ __forceinline__ void tc_panel(TcPanel& V, const Tc& T, bool have, const float* src, int ld, int row0, int c0,
+                                         int h, unsigned rm, int ident) {
+  const int tr = tc_tr(), kg = tc_kg();
+#pragma unroll
+  for (int half = 0; half < 2; half++)
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int col = 32 * half + 4 * kg;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (src) {
+        if ((rm >> i & 1) && col < h) v = *(const float4*)(src + (long long)(row0 + tr + 32 * i) * ld + c0 + col);
+      } else if (ident >= 0) {
+        const int j = row0 + tr + 32 * i - ident - col;
+        v.x = j == 0 ? 1.f : 0.f;
+        v.y = j == 1 ? 1.f : 0.f;
+        v.z = j == 2 ? 1.f : 0.f;
+        v.w = j == 3 ? 1.f : 0.f;
+      }
+      V.v[half][i] = v;
+    }
+  if (!have) return;
+  tc_drain(T);
+#pragma unroll
+  for (int half = 0; half < 2; half++)
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const float* e = T.Et + (tr + 32 * i) * kTcS + 32 * half + 4 * kg;
+      V.v[half][i].x -= e[0];
+      V.v[half][i].y -= e[1];
+      V.v[half][i].z -= e[2];
+      V.v[half][i].w -= e[3];
+    }
+}
+
+// D = V M^T over the rows in rm (M: h x h in Mt, zero outside), then dst rows row0 .., columns
+// c0 .. c0 + h = D; with out, also out[row ldo + col] = scale D.
+__device__ __forceinline__ bool tc_solve(Tc& T, const TcPanel& V, float* dst, int ld, int row0, int c0, int h,
+                                         unsigned rm, float* out = nullptr, int ldo = 0, float scale = 0.f) {
+  const int tr = tc_tr(), kg = tc_kg();
+  __syncthreads();  // every thread has read its part of Et
+#pragma unroll
+  for (int half = 0; half < 2; half++) {
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      tc_put(T.st.ahi, T.st.alo, tc_off(tr + 32 * i, kg),
+             (rm >> i & 1) ? V.v[half][i] : make_float4(0.f, 0.f, 0.f, 0.f));
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const float* m = T.Mt + (tr + 32 * i) * kTcS + 32 * half + 4 * kg;
+      tc_put(T.st.bhi, T.st.blo, tc_off(tr + 32 * i, kg),
+             tr + 32 * i < h ? make_float4(m[0], m[1], m[2], m[3]) : make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+    if (!tc_chunk(T, half == 0, [] {})) return false;
+  }
+  tc_drain(T);
+#pragma unroll
+  for (int half = 0; half < 2; half++)
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int col = 32 * half + 4 * kg, row = row0 + tr + 32 * i;
+      if (!(rm >> i & 1) || col >= h) continue;
+      const float* e = T.Et + (tr + 32 * i) * kTcS + col;
+      *(float4*)(dst + (long long)row * ld + c0 + col) = make_float4(e[0], e[1], e[2], e[3]);
+      if (out)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          if (col + j < h) out[(long long)row * ldo + col + j] = scale * e[j];
+    }
+  __syncthreads();
+  return true;
+}
+
+__global__ void __launch_bounds__(NTH, 3) k_chol_tc(int nblk, const int* __restrict__ blk_cell,
                                                      const long long* __restrict__ boff, const int* __restrict__ cs,
                                                      const long long* __restrict__ koff, float* __restrict__ K,
                                                      const long long* __restrict__ xoff, float* __restrict__ Xw,
@@ -876,34 +973,34 @@ __global__ void __launch_bounds__(NTH, 2) k_chol_tc(int nblk, const int* __restr
                                                      unsigned* __restrict__ err) {
   const int b = blockIdx.x;
   if (b >= nblk || (only && !only[b])) return;
-  constexpr int S = SP<float>::S;
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  float* base = (float*)smem_raw;
-  TcStage st;
-  st.ahi = base;
-  st.alo = st.ahi + 128 * TC_KCH;
-  st.bhi = st.alo + 128 * TC_KCH;
-  st.blo = st.bhi + 64 * TC_KCH;
-  float* Ct = st.blo + 64 * TC_KCH;  // [TB][S] diagonal tile
-  float* Mt = Ct + TB * S;           // [TB][S] its inverse
-  // epilogue staging of a 128 x 64 result, over the operand stage (48 KB >= 128 x 65 floats)
-  constexpr int kEtS = TB + 1;
-  static_assert(128 * kEtS <= 2 * 128 * TC_KCH + 2 * 64 * TC_KCH, "epilogue staging fits the operand stage");
-  float* Et = base;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t tmem_base;
   __shared__ int s_abort;
-  const int tid = threadIdx.x, w = tid >> 5;
+  const int tid = threadIdx.x, w = tid >> 5, tr = tc_tr(), kg = tc_kg();
+  Tc T;
+  T.st.ahi = (float*)smem_raw;
+  T.st.alo = T.st.ahi + TC_A;
+  T.st.bhi = T.st.alo + TC_A;
+  T.st.blo = T.st.bhi + TC_B;
+  T.Et = (float*)smem_raw;
+  T.Ct = T.Et + 128 * kTcS;
+  T.Mt = (float*)smem_raw + kTcStage;
+  T.bar = &bar;
+  T.s_abort = &s_abort;
+  T.err = err;
+  T.phase = 0;
 
+  // Rows and columns in memory: the n1 neighbour points, pad empty ones (S_c form), the n_c
+  // centre points. tile_range counts points; rows from n1 on move by pad.
   const int c = blk_cell[b];
-  const int nb = (int)(boff[c + 1] - boff[c]);
-  const int nc = cs[c + 1] - cs[c], n1 = mode == 1 ? nb : nb - nc;
+  const int np = (int)(boff[c + 1] - boff[c]);
+  const int nc = cs[c + 1] - cs[c], n1 = mode == 1 ? np : np - nc;
   const int kc1 = (n1 + TB - 1) / TB;
   const int ntile = kc1 + (mode == 1 ? 0 : (nc + TB - 1) / TB);
-  const int nct = ntile - kc1;
+  const int pad = mode == 1 ? 0 : tc_pad(n1), nb = np + pad, ld = tc_pitch(nb);
   float* A = K + koff[b];
   float* Minv_all = Xw + xoff[b];  // mode 0: the diagonal tiles' inverses, TB x TB each
-  (void)nct;
 
   if (tid == 0) {
     mbar_init(&bar, 1);
@@ -915,177 +1012,104 @@ __global__ void __launch_bounds__(NTH, 2) k_chol_tc(int nblk, const int* __restr
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   tc_sync();
-  const uint32_t tmem = tmem_base;
-  unsigned phase = 0;
-  bool ok = true;
-  const int r_own = 32 * (w & 3) + (tid & 31), cbase = 32 * (w >> 2);  // TMEM row / column half
+  T.tmem = tmem_base;
+  bool ok = true, run = true;
 
-  for (int k = 0; k < ntile && !s_abort; k++) {
+  for (int k = 0; k < ntile && run; k++) {
     int rk, hk;
-    tile_range(k, n1, nb, kc1, rk, hk);
-    for (int pr = rk; pr < nb && !s_abort; pr += 128) {
-      // ---- update: C = A[pr.., rk..] - sum over columns [0, rk) (rows pr .. pr + 127)
-      if (rk > 0) {
-        // next chunk's loads in flight while the tensor cores work on this one
-        TcRegs R;
-        tc_fetch(R, A, nb, pr, pr, nb, 0, rk, rk, rk + hk, nullptr, 0);
-        for (int c0 = 0; c0 < rk; c0 += TC_KCH) {
-          tc_store(st, R);
-          tc_sync();
-          if (tid == 0) tc_issue(tmem, st, c0 == 0);
-          if (c0 + TC_KCH < rk) tc_fetch(R, A, nb, pr, pr, nb, c0 + TC_KCH, rk, rk, rk + hk, nullptr, 0);
-          if (!tc_commit_wait(&bar, phase)) {
-            if (tid == 0) {
-              atomicOr(err, DEV_ERR_TIMEOUT);
-              s_abort = 1;
-            }
-          }
-          __syncthreads();
-          if (s_abort) break;
-        }
-        if (s_abort) break;
-        // the 128 x 64 update goes through shared memory (the operand stage, idle once the
-        // MMAs have committed), so the read-modify-write of the block is row-coalesced
-        {
-          float v[32];
-          tc_load32(tmem, v);
-#pragma unroll
-          for (int j = 0; j < 32; j++) Et[r_own * kEtS + cbase + j] = v[j];
-        }
-        __syncthreads();
-        // the diagonal tile keeps its lower part; rows below take the whole tile width. A
-        // thread's eight loads of the block are all issued before its first store (one
-        // load latency per eight entries instead of one per entry)
-        constexpr int kRmw = 8;
-        static_assert((128 * TB) % (kRmw * NTH) == 0, "whole groups");
-        for (int e0 = 0; e0 < 128 * TB; e0 += kRmw * NTH) {
-          float a[kRmw];
-#pragma unroll
-          for (int g = 0; g < kRmw; g++) {
-            const int e = e0 + g * NTH + tid, rr = e / TB, col = e % TB, row = pr + rr;
-            const bool in = row < nb && col < hk && (row >= rk + hk || col <= row - rk);
-            a[g] = in ? A[(long long)row * nb + rk + col] : 0.f;
-          }
-#pragma unroll
-          for (int g = 0; g < kRmw; g++) {
-            const int e = e0 + g * NTH + tid, rr = e / TB, col = e % TB, row = pr + rr;
-            if (row < nb && col < hk && (row >= rk + hk || col <= row - rk))
-              A[(long long)row * nb + rk + col] = a[g] - Et[rr * kEtS + col];
-          }
-        }
-        __syncthreads();
-      }
-      // ---- the diagonal tile (first panel of the column): factor and invert it
+    tile_range(k, n1, np, kc1, rk, hk);
+    if (k >= kc1) rk += pad;
+    for (int pr = rk; pr < nb && run; pr += 128) {
+      // ---- update: V = A[pr.., rk..] - sum over columns [0, rk) (rows pr .. pr + 127)
+      if (rk > 0) run = tc_sum<false>(T, A, ld, pr, nb, A, rk, hk, 0, rk);
+      if (!run) break;
+      TcPanel V;
+      tc_panel(V, T, rk > 0, A, ld, pr, rk, hk, tc_rows(pr, 0, nb), -1);
+      // ---- the diagonal tile (first panel of the column): factor and invert it; the rows
+      // below it wait in Et
       if (pr == rk) {
-        for (int e = tid; e < TB * TB; e += NTH) {
-          const int r = e / TB, cc = e % TB;
-          Ct[r * S + cc] = (r < hk && cc <= r) ? A[(long long)(rk + r) * nb + rk + cc] : 0.f;
-        }
-        __syncthreads();
-        ok = potrf_trtri_w(Ct, Mt, hk) && ok;
-        for (int e = tid; e < TB * TB; e += NTH) {
-          const int r = e / TB, cc = e % TB;
-          if (r < hk && cc <= r) A[(long long)(rk + r) * nb + rk + cc] = Ct[r * S + cc];
-          if (mode == 0) Minv_all[(long long)k * TB * TB + e] = Mt[r * S + cc];
-        }
-        __syncthreads();
-      }
-      // ---- panel solve of the rows below the diagonal tile: L = C M^T (M = L_kk^-1)
-      if (pr + 128 > rk + hk && rk + hk < nb) {
-        TcRegs R;
-        for (int c0 = 0; c0 < TB; c0 += TC_KCH) {
-          tc_fetch(R, A, nb, pr, rk + hk, nb, rk + c0, rk + hk, 0, hk, Mt, c0);
-          tc_store(st, R);
-          tc_sync();
-          if (tid == 0) tc_issue(tmem, st, c0 == 0);
-          if (!tc_commit_wait(&bar, phase)) {
-            if (tid == 0) {
-              atomicOr(err, DEV_ERR_TIMEOUT);
-              s_abort = 1;
+#pragma unroll
+        for (int half = 0; half < 2; half++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const int r = tr + 32 * i, col = 32 * half + 4 * kg;
+            const float* v = (const float*)&V.v[half][i];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              T.Et[r * kTcS + col + j] = v[j];
+              if (i < 2) T.Ct[r * kTcS + col + j] = (r < hk && col + j <= r) ? v[j] : 0.f;
             }
           }
-          __syncthreads();
-          if (s_abort) break;
-        }
-        if (s_abort) break;
-        {
-          float v[32];
-          tc_load32(tmem, v);
-#pragma unroll
-          for (int j = 0; j < 32; j++) Et[r_own * kEtS + cbase + j] = v[j];
-        }
-        __syncthreads();  // every thread has read its C row and staged its result
-        for (int e = tid; e < 128 * TB; e += NTH) {
-          const int rr = e / TB, col = e % TB, row = pr + rr;
-          if (row < nb && row >= rk + hk && col < hk) A[(long long)row * nb + rk + col] = Et[rr * kEtS + col];
-        }
         __syncthreads();
+        ok = potrf_trtri_w(T.Ct, T.Mt, hk) && ok;
+#pragma unroll
+        for (int half = 0; half < 2; half++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const int r = tr + 32 * i, col = 32 * half + 4 * kg;
+            if (i < 2) {
+              const float* e = T.Ct + r * kTcS + col;
+              if (r < hk && col <= r)
+                *(float4*)(A + (long long)(rk + r) * ld + rk + col) = make_float4(e[0], e[1], e[2], e[3]);
+              const float* m = T.Mt + r * kTcS + col;
+              if (mode == 0)
+                *(float4*)(Minv_all + (long long)k * TB * TB + r * TB + col) = make_float4(m[0], m[1], m[2], m[3]);
+            }
+            const float* e = T.Et + r * kTcS + col;
+            V.v[half][i] = make_float4(e[0], e[1], e[2], e[3]);
+          }
       }
+      // ---- panel solve of the rows below the diagonal tile: L = V M^T (M = L_kk^-1)
+      if (pr + 128 > rk + hk && rk + hk < nb)
+        run = tc_solve(T, V, A, ld, pr, rk, hk, tc_rows(pr, rk + hk, nb));
+      else
+        __syncthreads();
     }
   }
 
   // ---- S_c = 2 pi sigma^2 X^T, X the centre columns of K^-1 (mode 0) --------------------
-  // Z = X^T (n_c x n_b, row-major, written in place at S_c) solves Z L L^T = E_c^T, E_c the
-  // centre columns of the identity. Forward, over the centre tiles I only (Z is zero left
-  // of them): Z_I = (E_I^T - Z[:, n1..r_I) L_I,[n1..r_I)^T) M_II^T. Back, over all tiles
-  // from the last: Z_J = (Z_J - Z[:, r_J + h_J..) (L^T)_J,[r_J + h_J..)^T) M_JJ with the rows
-  // of L^T read as columns of L (transposed fetch). Every product is a 128-row panel of Z (128
-  // centre points per pass) times 64 rows of L, L^T or M on the tensor cores, the same MMA pipeline
-  // as the factorisation. The centre columns are scaled once they are final; the neighbour
-  // columns, linear in them, then come out scaled.
-  if (mode == 0 && ok && !s_abort) {
-    float* Z = Sout + soff[c];
+  // Z = X^T / (2 pi sigma^2) (n_c rows at the block's pitch, behind the inverses) solves
+  // Z L L^T = E_c^T, E_c the centre columns of the identity. Forward, over the centre tiles I
+  // only (Z is zero left of them): Z_I = (E_I^T - Z[:, n1..r_I) L_I,[n1..r_I)^T) M_II^T. Back,
+  // over all tiles from the last: Z_J = (Z_J - Z[:, r_J + h_J..) (L^T)_J,[r_J + h_J..)^T) M_JJ
+  // with the rows of L^T read as columns of L (transposed fetch), written to Z and, scaled, to
+  // S_c. Every product is a 128-row panel of Z (128 centre points per pass) times 64 rows of L,
+  // L^T or M on the tensor cores, the same MMA pipeline as the factorisation.
+  if (mode == 0 && ok && run) {
+    float* Z = Minv_all + (long long)ntile * TB * TB;
+    float* S = Sout + soff[c];
     const float zscale = (float)(cell_sig ? 2.0 * M_PI * cell_sig[c] * cell_sig[c] : out_scale_all);
-    for (int n = w; n < nc; n += NTH / 32) {  // a warp per row of Z
-      float* zr = Z + (long long)n * nb;
-      for (int j = tid & 31; j < nb; j += 32) zr[j] = j == n1 + n ? 1.f : 0.f;
-    }
-    __syncthreads();
-    for (int pr = 0; pr < nc && !s_abort; pr += 128) {
-      for (int I = kc1; I < ntile && !s_abort; I++) {  // forward
-        int rI, hI;
-        tile_range(I, n1, nb, kc1, rI, hI);
-        if (rI > n1) {
-          if (!tc_gemm(st, tmem, &bar, phase, &s_abort, err, Z, nb, pr, pr, nc, A, rI, rI + hI, nullptr, n1, rI))
-            break;
-          tc_epi(tmem, Et, Z, nb, pr, nc, rI, hI, true);
+    const int nz = n1 + pad;  // the first centre column
+    for (int pr = 0; pr < nc && run; pr += 128) {
+      const unsigned rm = tc_rows(pr, 0, nc);
+      for (int st = 0; st < ntile - kc1 + ntile && run; st++) {
+        const bool fwd = st < ntile - kc1;
+        const int J = fwd ? kc1 + st : 2 * ntile - kc1 - 1 - st;
+        int r0, h;
+        tile_range(J, n1, np, kc1, r0, h);
+        const int rJ = J < kc1 ? r0 : r0 + pad, k1 = J == kc1 - 1 ? nz : rJ + h;  // k1: the next tile's column
+        const bool have = fwd ? rJ > nz : k1 < nb;
+        // M_JJ, or its transpose in the back pass
+        for (int u = tid; u < TB * TB / 4; u += NTH) {
+          const int r = u / (TB / 4), col = 4 * (u % (TB / 4));
+          const float4 m = *(const float4*)(Minv_all + (long long)J * TB * TB + 4 * u);
+          const float mv[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+          for (int j = 0; j < 4; j++) T.Mt[fwd ? r * kTcS + col + j : (col + j) * kTcS + r] = mv[j];
         }
-        for (int e = tid; e < TB * TB; e += NTH) Mt[(e / TB) * S + e % TB] = Minv_all[(long long)I * TB * TB + e];
-        __syncthreads();
-        if (!tc_gemm(st, tmem, &bar, phase, &s_abort, err, Z, nb, pr, pr, nc, nullptr, 0, hI, Mt, rI, rI + hI)) break;
-        tc_epi(tmem, Et, Z, nb, pr, nc, rI, hI, false);
-      }
-      for (int J = ntile - 1; J >= 0 && !s_abort; J--) {  // back
-        int rJ, hJ;
-        tile_range(J, n1, nb, kc1, rJ, hJ);
-        if (J == kc1 - 1) {  // the centre columns are final: scale them
-          for (int n = pr + w; n < min(pr + 128, nc); n += NTH / 32)
-            for (int j = n1 + (tid & 31); j < nb; j += 32) Z[(long long)n * nb + j] *= zscale;
-          __syncthreads();
-        }
-        if (rJ + hJ < nb) {
-          if (!tc_gemm(st, tmem, &bar, phase, &s_abort, err, Z, nb, pr, pr, nc, A, rJ, rJ + hJ, nullptr, rJ + hJ, nb,
-                       true))
-            break;
-          tc_epi(tmem, Et, Z, nb, pr, nc, rJ, hJ, true);
-        }
-        for (int e = tid; e < TB * TB; e += NTH)  // M_JJ^T
-          Mt[(e % TB) * S + e / TB] = Minv_all[(long long)J * TB * TB + e];
-        __syncthreads();
-        if (!tc_gemm(st, tmem, &bar, phase, &s_abort, err, Z, nb, pr, pr, nc, nullptr, 0, hJ, Mt, rJ, rJ + hJ)) break;
-        tc_epi(tmem, Et, Z, nb, pr, nc, rJ, hJ, false);
-      }
-      if (kc1 == 0 && !s_abort) {  // no neighbour tiles: the centre columns are all of Z
-        for (int n = pr + w; n < min(pr + 128, nc); n += NTH / 32)
-          for (int j = n1 + (tid & 31); j < nb; j += 32) Z[(long long)n * nb + j] *= zscale;
-        __syncthreads();
+        if (have)
+          run = fwd ? tc_sum<false>(T, Z, ld, pr, nc, A, rJ, h, nz, rJ) : tc_sum<true>(T, Z, ld, pr, nc, A, rJ, h, k1, nb);
+        if (!run) break;
+        TcPanel V;
+        tc_panel(V, T, have, !fwd && J >= kc1 ? Z : nullptr, ld, pr, rJ, h, rm, fwd ? rJ - nz : -1);
+        run = tc_solve(T, V, Z, ld, pr, rJ, h, rm, fwd ? nullptr : S + r0, np, zscale);
       }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (w == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(64));
-  if (tid == 0) bad[b] = (ok && !s_abort) ? 0 : 1;
+  if (w == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(T.tmem), "r"(64));
+  if (tid == 0) bad[b] = (ok && run) ? 0 : 1;
 }
 
 // After k_chol_tc (factor form): each block's L packed by rows as the substitutions read
@@ -1106,11 +1130,11 @@ __global__ void __launch_bounds__(NTH) k_pack_factor(int nblk, const int* __rest
   const float sc = (float)(cell_sig ? sqrt(1.0 / (2.0 * M_PI * cell_sig[c] * cell_sig[c])) : scale_all);
   const float* A = K + koff[b];
   float* Lp = Lpack + loff[c];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, ld = tc_pitch(nb);
   for (int i = w; i < nb; i += NTH / 32) {
     const long long o = rowoff<float>(i);
     for (int j = lane; j <= i; j += 32) {
-      const float v = A[(long long)i * nb + j] * sc;
+      const float v = A[(long long)i * ld + j] * sc;
       Lp[o + j] = j == i ? 1.f / v : v;
     }
   }
@@ -1945,7 +1969,7 @@ void rasm_block_K(const RasmPlan& R, const PointSet& P, int cell, int nb, double
   k_assemble<double><<<dim3(64, 1), 256, 0, s>>>(1, dbc, R.boff.get(), P.cs.get(), R.idx.get(), dk, P.x.get(),
                                                   P.y.get(), P.view().z, g.dim, 1.0 / (2.0 * g.sigma * g.sigma),
                                                   nullptr, 0.0, K_dev, nullptr, nullptr, 0, kexp_of_sigma(g.sigma),
-                                                  exp_table_dev(s));
+                                                  exp_table_dev(s), 0);
   PRBF_CHECK_LAUNCH();
   PRBF_CUDA(cudaStreamSynchronize(s));  // the host copies of dbc / dk stay valid until here
 }
@@ -2003,7 +2027,7 @@ void lu_build(RasmPlan& R, const BlockGeom& G, const std::vector<int>& hcnt, std
     k_assemble<double><<<dim3(64, m), 256, 0, s>>>(m, R.lucell.get() + b0, R.boff.get(), G.cs, R.idx.get(),
                                                    R.lukoff.get() + b0, G.x, G.y, G.z, G.dim, inv2s2, G.cell_sigma,
                                                    0.0, R.LU64.get(), nullptr, nullptr, 0, kexp_of_sigma(G.sigma),
-                                                   exp_table_dev(s));
+                                                   exp_table_dev(s), 0);
     PRBF_CHECK_LAUNCH();
   }
   unsigned char* dbad = (unsigned char*)ws.get(50, nlu);
@@ -2133,7 +2157,12 @@ void rasm_factor(RasmPlan& R, const BlockGeom& G, const std::vector<int>& hcnt, 
       long long nbk = hcnt[c], nc = hcs[c + 1] - hcs[c];
       long long n1 = nbk - nc;
       long long ntile = (n1 + TB - 1) / TB + (nc + TB - 1) / TB;
-      long long ke = nbk * nbk, xe = R.factor ? 1 : ntile * TB * TB;  // S_c form: FP32 only
+      long long ke = nbk * nbk, xe = 1;
+      if (fp32) {  // the tensor-core form's pitch; S_c form: the diagonal inverses and Z
+        const long long nbp = nbk + (R.factor ? 0 : tc_pad((int)n1));
+        ke = nbp * tc_pitch((int)nbp);
+        if (!R.factor) xe = ntile * TB * TB + nc * tc_pitch((int)nbp);
+      }
       if (!bc.empty() && (double)(hk.back() + ke + hx.back() + xe) * esz > ws_budget_bytes) break;
       if (bc.size() >= 65535) break;  // gridDim.y of the assembly
       bc.push_back(c);
@@ -2159,7 +2188,7 @@ void rasm_factor(RasmPlan& R, const BlockGeom& G, const std::vector<int>& hcnt, 
       if (fp32) {
         k_assemble<float><<<ag, 256, asm_smem, s>>>(nb_batch, dbc, R.boff.get(), G.cs, R.idx.get(), dk, G.x, G.y, G.z, G.dim,
                                              inv2s2, G.cell_sigma, shift, (float*)Kw, only, hl, (long long)G.n,
-                                             0.0, nullptr);
+                                             0.0, nullptr, R.factor ? 0 : 1);
         PRBF_CHECK_LAUNCH();
         // the Cholesky on the tensor cores (and S_c), then the packed factor
         k_chol_tc<<<nb_batch, NTH, chol_tc_smem(), s>>>(nb_batch, dbc, R.boff.get(), G.cs, dk, (float*)Kw, dx,
@@ -2174,7 +2203,7 @@ void rasm_factor(RasmPlan& R, const BlockGeom& G, const std::vector<int>& hcnt, 
       } else {
         k_assemble<double><<<ag, 256, 0, s>>>(nb_batch, dbc, R.boff.get(), G.cs, R.idx.get(), dk, G.x, G.y, G.z,
                                               G.dim, inv2s2, G.cell_sigma, shift, (double*)Kw, only, nullptr, 0,
-                                              kexp_of_sigma(G.sigma), exp_table_dev(s));
+                                              kexp_of_sigma(G.sigma), exp_table_dev(s), 0);
         PRBF_CHECK_LAUNCH();
         const int ncl = chol_cluster(nb_batch);
         cudaLaunchConfig_t cfg = {};
