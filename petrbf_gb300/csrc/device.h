@@ -151,13 +151,14 @@ struct GaussPlan {
   DevBuf<int2> sym_items;
 };
 
-// The forms of the sum a plan is used for: the FP32 products, the FP64 products (neither for
-// a plan used only for its sizes).
-enum : int { FORM_F32 = 1, FORM_F64 = 2 };
-// Builds the work list and the truncation-set sizes; sets plan.pairs / max_trunc, and the
-// point data of the forms asked for.
+// What a plan is used for: the FP32 products, the FP64 products (neither for a plan used only
+// for its sizes), the truncation-set sizes (trunc_cnt, pairs, max_trunc; zero when not asked
+// for -- a single evaluation has no use for them, and they are 200 us of 1.7 ms at 5x10^5
+// sources and 3x10^5 targets).
+enum : int { FORM_F32 = 1, FORM_F64 = 2, PLAN_COUNTS = 4 };
+// Builds the work list, the truncation-set sizes and the point data as asked for.
 void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& src,
-                    unsigned* err, Workspace& ws, cudaStream_t s, int forms = FORM_F32 | FORM_F64);
+                    unsigned* err, Workspace& ws, cudaStream_t s, int forms = FORM_F32 | FORM_F64 | PLAN_COUNTS);
 // Point data of a batch (plan.grids and plan.cprob set: each problem with its own grid and
 // scale, grids with their first global cell); sets plan.f32_ready / fx_ready for the forms
 // asked for when every grid qualifies.

@@ -1315,20 +1315,26 @@ __global__ void __launch_bounds__(kThreads) k_gauss_sym(
   }
 }
 
-// Rows += their partial slots (offset order), slots back to zero for the next product.
+// Rows += their partial slots (offset order), slots back to zero for the next product. A batch's
+// loads are issued before its stores: 10^4 points (24 slots) are bound by that chain's latency.
+constexpr int kGatherBatch = 8;
 __global__ void k_sym_gather(int n, int nv, int K, long long pstride, double* __restrict__ part,
                              double* __restrict__ w, long long vs, const int* __restrict__ skip) {
   if (skip && *skip) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     for (int v = 0; v < nv; v++) {
       double s = 0.0;
-      for (int o = 0; o < K; o++) {
-        double* slot = part + ((long long)v * K + o) * pstride + i;
-        const double x = *slot;
-        if (__double_as_longlong(x) != 0) {  // an integer test: the FP64 pipe is for the sums
-          s += x;
-          *slot = 0.0;
-        }
+      for (int o0 = 0; o0 < K; o0 += kGatherBatch) {
+        double* slot = part + ((long long)v * K + o0) * pstride + i;
+        double x[kGatherBatch];
+#pragma unroll
+        for (int o = 0; o < kGatherBatch; o++) x[o] = o0 + o < K ? slot[o * pstride] : 0.0;
+#pragma unroll
+        for (int o = 0; o < kGatherBatch; o++)
+          if (__double_as_longlong(x[o]) != 0) {  // an integer test: the FP64 pipe is for the sums
+            s += x[o];
+            slot[o * pstride] = 0.0;
+          }
       }
       w[v * vs + i] += s;
     }
@@ -1666,20 +1672,22 @@ void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& sr
   plan.items.reserve(std::max(nitems, 1));
   k_item_fill<<<ceil_div(g.ncell, 256), 256, 0, s>>>(g.ncell, tgt.cell_start, cnt, plan.items.get());
   PRBF_CHECK_LAUNCH();
-  plan.trunc_cnt.reserve(g.ncell);
   struct {
     unsigned long long pairs;
     int maxc;
     int pad;
   } h{0, 0, 0};
-  void* d = ws.get(24, sizeof(h));
-  PRBF_CUDA(cudaMemsetAsync(d, 0, sizeof(h), s));
-  k_trunc_count<<<ceil_div(g.ncell, 8), 256, 0, s>>>(g, tgt.cell_start, src.x, src.y, src.z,
-                                                     src.cell_start, plan.trunc_cnt.get(),
-                                                     (unsigned long long*)d, (int*)((char*)d + 8));
-  PRBF_CHECK_LAUNCH();
-  PRBF_CUDA(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, s));
-  PRBF_CUDA(cudaStreamSynchronize(s));
+  if (forms & PLAN_COUNTS) {
+    plan.trunc_cnt.reserve(g.ncell);
+    void* d = ws.get(24, sizeof(h));
+    PRBF_CUDA(cudaMemsetAsync(d, 0, sizeof(h), s));
+    k_trunc_count<<<ceil_div(g.ncell, 8), 256, 0, s>>>(g, tgt.cell_start, src.x, src.y, src.z,
+                                                       src.cell_start, plan.trunc_cnt.get(),
+                                                       (unsigned long long*)d, (int*)((char*)d + 8));
+    PRBF_CHECK_LAUNCH();
+    PRBF_CUDA(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, s));
+    PRBF_CUDA(cudaStreamSynchronize(s));
+  }
   plan.pairs = (long long)h.pairs;
   plan.max_trunc = h.maxc;
   plan.max_tile = kTileT;
@@ -1688,7 +1696,7 @@ void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& sr
   plan.sym_ready = false;
   plan.sym_nitems = 0;
   plan.sym_ncs = 0;
-  if (!forms) return;
+  if (!(forms & (FORM_F32 | FORM_F64))) return;
   const bool self = tgt.x == src.x && tgt.n == src.n;
   if (f32_grid_ok(g) && src.n > 0) {
     const bool f32 = forms & FORM_F32, fx = (forms & FORM_F64) && fx_grid_ok(g);

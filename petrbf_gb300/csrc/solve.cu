@@ -116,7 +116,7 @@ static void interpolate(Ctx& c, int n, const double* x, const double* y, const d
   S.plan.sym_nv = std::min(4, nrhs);  // right-hand sides summed together by the symmetric form
   const bool mixed = p.precision == PRBF_PREC_MIXED;
   gauss_plan_dev(S.plan, S.pts.view(), S.pts.view(), c.err.get(), c.ws, c.stream,
-                 FORM_F64 | (mixed ? FORM_F32 : 0));
+                 PLAN_COUNTS | FORM_F64 | (mixed ? FORM_F32 : 0));
   size_t free_b = 0, total_b = 0;
   PRBF_CUDA(cudaMemGetInfo(&free_b, &total_b));
   double budget = std::min(16.0e9, 0.25 * (double)free_b);
