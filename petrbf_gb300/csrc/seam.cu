@@ -18,6 +18,7 @@
 //
 // Device buffers are grow-only and held for the life of the process, one set per device,
 // as the reference's file statics are (2d/gpumatmult.cu:7-18); calls are serialised.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -45,12 +46,12 @@ __global__ void __launch_bounds__(kSlots) k_seam(const int* __restrict__ offset,
                                                  float* __restrict__ tw, float c2, double norm,
                                                  const float* __restrict__ sx, const float* __restrict__ sy,
                                                  const float* __restrict__ sz, const float* __restrict__ sg,
-                                                 unsigned* err) {
+                                                 unsigned* err, int b0) {
   constexpr int NA = DIM + 1;  // staged arrays: coordinates + weight
   __shared__ __align__(16) float buf[2][NA][kRow];
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ int s_abort;
-  const int b = blockIdx.x, t = threadIdx.x;
+  const int b = b0 + blockIdx.x, t = threadIdx.x;
   const long long i = (long long)b * kSlots + t;
   const float x = tx[i], y = ty[i], z = DIM == 3 ? tz[i] : 0.f;
   const int j0 = offset[b], j1 = offset[b + 1];
@@ -126,9 +127,19 @@ __global__ void __launch_bounds__(kSlots) k_seam(const int* __restrict__ offset,
   tw[i] = (float)((double)acc * norm);
 }
 
+// The sources (12 to 16 bytes each) take longer to arrive than to sum, so a call is cut into
+// parts of whole blocks of about equal source counts: a part's kernel runs on a second stream
+// while the next part's sources are copied. A copy from pageable memory costs some 15 us by
+// itself, which bounds the number of parts. 2D, the whole call with 1 / 2 / 3 / 4 / 8 parts:
+// 4.33e6 sources 612 / 575 / 592 / 609 / 723 us; 8.88e6 sources 1145 / 1054 / 1033 / 1066 /
+// 1135 us.
+constexpr int kMaxParts = 3;
+constexpr long long kPartSources = 1 << 21;  // sources of a part at least
+
 struct SeamBufs {
   std::mutex m;
-  cudaStream_t s = nullptr;
+  cudaStream_t s = nullptr, k = nullptr;  // copies; kernels and the result's copy
+  cudaEvent_t in[kMaxParts] = {nullptr};  // a part's sources have arrived
   DevBuf<int> off;
   DevBuf<float> t[4], src[4];
   DevBuf<unsigned> err;
@@ -165,7 +176,12 @@ int seam(const float* tX, const float* tY, const float* tZ, float* tW, const flo
     PRBF_CUDA(cudaGetDevice(&dev));
     SeamBufs& S = seam_bufs(dev);
     std::lock_guard<std::mutex> lk(S.m);
-    if (!S.s) PRBF_CUDA(cudaStreamCreateWithFlags(&S.s, cudaStreamNonBlocking));
+    if (!S.s) {
+      for (cudaEvent_t& e : S.in)
+        if (!e) PRBF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      if (!S.k) PRBF_CUDA(cudaStreamCreateWithFlags(&S.k, cudaStreamNonBlocking));
+      PRBF_CUDA(cudaStreamCreateWithFlags(&S.s, cudaStreamNonBlocking));
+    }
     const long long nt = (long long)iblok * kSlots;
     S.off.reserve((size_t)iblok + 1);
     for (int a = 0; a < (DIM == 3 ? 4 : 3); a++) S.t[a].reserve((size_t)nt);
@@ -173,30 +189,53 @@ int seam(const float* tX, const float* tY, const float* tZ, float* tW, const flo
     const size_t ns_alloc = (size_t)nsrc + 8;
     for (int a = 0; a < (DIM == 3 ? 4 : 3); a++) S.src[a].reserve(ns_alloc);
     S.err.reserve(1);
+    // nothing of this call is left in flight when it fails: the caller's arrays and the buffers
+    // are the next call's
+    struct Drain {
+      SeamBufs& S;
+      ~Drain() {
+        cudaStreamSynchronize(S.s);
+        cudaStreamSynchronize(S.k);
+      }
+    } drain{S};
     PRBF_CUDA(cudaMemsetAsync(S.err.get(), 0, sizeof(unsigned), S.s));
     PRBF_CUDA(cudaMemcpyAsync(S.off.get(), offset, sizeof(int) * ((size_t)iblok + 1), cudaMemcpyHostToDevice, S.s));
     const float* th[3] = {tX, tY, tZ};
     for (int a = 0; a < DIM; a++)
       PRBF_CUDA(cudaMemcpyAsync(S.t[a].get(), th[a], sizeof(float) * nt, cudaMemcpyHostToDevice, S.s));
     const float* sh[4] = {sX, sY, DIM == 3 ? sZ : sG, sG};
-    for (int a = 0; a <= DIM; a++) {
-      float* d = S.src[a].get();
-      if (nsrc > 0) PRBF_CUDA(cudaMemcpyAsync(d, sh[a], sizeof(float) * nsrc, cudaMemcpyHostToDevice, S.s));
-      PRBF_CUDA(cudaMemsetAsync(d + nsrc, 0, sizeof(float) * 8, S.s));
-    }
+    for (int a = 0; a <= DIM; a++) PRBF_CUDA(cudaMemsetAsync(S.src[a].get() + nsrc, 0, sizeof(float) * 8, S.s));
     // coef = 0.5 / sigma^2 (2d/gpumatmult.cu:33); exp(-d2 coef) = 2^(-d2 coef log2 e)
     const double coef = 0.5 / ((double)sigma * (double)sigma);
     const float c2 = (float)(coef * 1.4426950408889634);
     const double norm = coef / 3.141592653589793;
     float* tw_dev = S.t[DIM].get();
-    k_seam<DIM><<<iblok, kSlots, 0, S.s>>>(S.off.get(), S.t[0].get(), S.t[1].get(), DIM == 3 ? S.t[2].get() : nullptr,
-                                           tw_dev, c2, norm, S.src[0].get(), S.src[1].get(),
-                                           DIM == 3 ? S.src[2].get() : nullptr, S.src[DIM].get(), S.err.get());
-    PRBF_CHECK_LAUNCH();
+    const int parts = (int)std::max(1LL, std::min<long long>(kMaxParts, nsrc / kPartSources));
+    long long c0 = 0;  // sources copied so far
+    for (int p = 0, b0 = 0; p < parts && b0 < iblok; p++) {
+      // blocks [b0, b1); their sources, and the up to three of the next block that share the
+      // last 16 bytes a chunk's copy reads
+      int b1 = iblok;
+      if (p + 1 < parts)
+        b1 = (int)(std::lower_bound(offset + b0 + 1, offset + iblok, (int)(nsrc * (p + 1) / parts)) - offset);
+      const long long c1 = std::min(nsrc, ((long long)offset[b1] + 3) & ~3LL);
+      for (int a = 0; a <= DIM && c1 > c0; a++)
+        PRBF_CUDA(cudaMemcpyAsync(S.src[a].get() + c0, sh[a] + c0, sizeof(float) * (c1 - c0), cudaMemcpyHostToDevice,
+                                  S.s));
+      PRBF_CUDA(cudaEventRecord(S.in[p], S.s));
+      PRBF_CUDA(cudaStreamWaitEvent(S.k, S.in[p], 0));
+      k_seam<DIM><<<b1 - b0, kSlots, 0, S.k>>>(S.off.get(), S.t[0].get(), S.t[1].get(),
+                                               DIM == 3 ? S.t[2].get() : nullptr, tw_dev, c2, norm, S.src[0].get(),
+                                               S.src[1].get(), DIM == 3 ? S.src[2].get() : nullptr, S.src[DIM].get(),
+                                               S.err.get(), b0);
+      PRBF_CHECK_LAUNCH();
+      c0 = std::max(c0, c1);
+      b0 = b1;
+    }
     unsigned herr = 0;
-    PRBF_CUDA(cudaMemcpyAsync(tW, tw_dev, sizeof(float) * nt, cudaMemcpyDeviceToHost, S.s));
-    PRBF_CUDA(cudaMemcpyAsync(&herr, S.err.get(), sizeof(unsigned), cudaMemcpyDeviceToHost, S.s));
-    PRBF_CUDA(cudaStreamSynchronize(S.s));
+    PRBF_CUDA(cudaMemcpyAsync(tW, tw_dev, sizeof(float) * nt, cudaMemcpyDeviceToHost, S.k));
+    PRBF_CUDA(cudaMemcpyAsync(&herr, S.err.get(), sizeof(unsigned), cudaMemcpyDeviceToHost, S.k));
+    PRBF_CUDA(cudaStreamSynchronize(S.k));
     if (herr) return PRBF_ERR_TIMEOUT;
     return PRBF_OK;
   } catch (const Error& e) {
