@@ -1715,11 +1715,11 @@ __global__ void __launch_bounds__(kTrwWarps * 32) k_apply_trw(int ncell, const l
     double* Yc = Y + boff[c];
     for (int j = lane; j < nb; j += 32)
 #pragma unroll
-      for (int v = 0; v < NV; v++) Yc[v * ys + (j < n1 ? nc + j : j - n1)] = (double)y[v * ldy + j];
+      for (int v = 0; v < NV; v++) Yc[vm[v] * ys + (j < n1 ? nc + j : j - n1)] = (double)y[v * ldy + j];
   } else {
     for (int i = lane; i < nc; i += 32)
 #pragma unroll
-      for (int v = 0; v < NV; v++) out[v * vs + cs[c] + i] = (double)y[v * ldy + n1 + i];
+      for (int v = 0; v < NV; v++) out[vm[v] * vs + cs[c] + i] = (double)y[v * ldy + n1 + i];
   }
 }
 
