@@ -1,7 +1,7 @@
 // devpool.cu -- device memory kept between uses. A cudaMalloc and cudaFree pair costs 60 us
 // (430 us at 512 MB), and a one-shot call (its own context, some thirty buffers) spent most of its
 // time in them: evaluating 4.9x10^5 sources at 3x10^5 points took 3.6 ms, 1.4 of them kernels, and
-// takes 1.7 now; the 10^4-point solve in a context of its own 35.4 -> 34.3 ms.
+// 1.7 with the pool; the 10^4-point solve in a context of its own 35.4 -> 34.3 ms.
 //
 // A freed block may still be read by work its stream has queued, so it carries that stream (the
 // context's, set for the length of a call, StreamScope) and serves the same stream again at once,

@@ -1316,7 +1316,8 @@ __global__ void __launch_bounds__(kThreads) k_gauss_sym(
 }
 
 // Rows += their partial slots (offset order), slots back to zero for the next product. A batch's
-// loads are issued before its stores: 10^4 points (24 slots) are bound by that chain's latency.
+// loads are issued before its stores: small products (2500 points, 24 slots) are bound by that
+// chain's latency.
 constexpr int kGatherBatch = 8;
 __global__ void k_sym_gather(int n, int nv, int K, long long pstride, double* __restrict__ part,
                              double* __restrict__ w, long long vs, const int* __restrict__ skip) {

@@ -15,7 +15,7 @@
 // stay in registers; their lanes stride over a buffer's sources. Nothing but the buffers' mbarriers joins the warps: with CTA barriers around the
 // filtering they spent a fifth of their time waiting there.
 // Measured against the FP64-pipe kernels of gauss.cu (one product, caller order): 2D, 4x10^6
-// points 44.7 -> 8.1 ms (79.8 -> 440 Gpairs/s); 3D, 96^3 points 180.7 -> 18.7 ms (39.5 -> 381).
+// points 44.7 -> 7.9 ms (79.8 -> 450 Gpairs/s); 3D, 96^3 points 180.7 -> 18.7 ms (39.5 -> 381).
 // What bounds it: the FP64 accumulations take 16 of the 23 (2D) to 27 (3D) clocks an SM spends
 // per 32 pairs; the shared-memory lookups (14), the integer pipes (10 to 13) and the issue of
 // about 50 instructions (12) overlap with them, 24 warps an SM not hiding all of it.
