@@ -349,7 +349,9 @@ def run_ours(args, rank, world):
                      "flops_per_pair": FLOPS_PER_PAIR,
                      "symmetric": symmetric,
                      "note": ("achieved counts the reference's 15 flops per ordered pair; the symmetric sum "
-                              "evaluates one exponential for both ordered pairs of a point pair") if symmetric else None,
+                              "evaluates one exponential for both ordered pairs of a point pair, in fixed point on "
+                              "the integer pipes, so the FP64 pipe is left one FMA per ordered pair and the "
+                              "fraction exceeds one") if symmetric else None,
                      "traffic": profile_traffic("gauss_fp64_2d_N4e6.txt"),
                      "hbm_view": hbm_view(32 * n, ms / args.steps)},
         "fp32_matvec_gpairs": fp32_gpairs,
