@@ -132,7 +132,8 @@ __global__ void __launch_bounds__(kSlots) k_seam(const int* __restrict__ offset,
 // while the next part's sources are copied. A copy from pageable memory costs some 15 us by
 // itself, which bounds the number of parts. 2D, the whole call with 1 / 2 / 3 / 4 / 8 parts:
 // 4.33e6 sources 612 / 575 / 592 / 609 / 723 us; 8.88e6 sources 1145 / 1054 / 1033 / 1066 /
-// 1135 us.
+// 1135 us. Below 2^22 sources there is one part and one stream (a second one, with its event,
+// costs 5 us of a call of 114).
 constexpr int kMaxParts = 3;
 constexpr long long kPartSources = 1 << 21;  // sources of a part at least
 
@@ -193,11 +194,13 @@ int seam(const float* tX, const float* tY, const float* tZ, float* tW, const flo
     // are the next call's
     struct Drain {
       SeamBufs& S;
+      bool armed;
       ~Drain() {
+        if (!armed) return;
         cudaStreamSynchronize(S.s);
         cudaStreamSynchronize(S.k);
       }
-    } drain{S};
+    } drain{S, true};
     PRBF_CUDA(cudaMemsetAsync(S.err.get(), 0, sizeof(unsigned), S.s));
     PRBF_CUDA(cudaMemcpyAsync(S.off.get(), offset, sizeof(int) * ((size_t)iblok + 1), cudaMemcpyHostToDevice, S.s));
     const float* th[3] = {tX, tY, tZ};
@@ -211,6 +214,7 @@ int seam(const float* tX, const float* tY, const float* tZ, float* tW, const flo
     const double norm = coef / 3.141592653589793;
     float* tw_dev = S.t[DIM].get();
     const int parts = (int)std::max(1LL, std::min<long long>(kMaxParts, nsrc / kPartSources));
+    const cudaStream_t ks = parts > 1 ? S.k : S.s;  // (one part: no second stream, no event)
     long long c0 = 0;  // sources copied so far
     for (int p = 0, b0 = 0; p < parts && b0 < iblok; p++) {
       // blocks [b0, b1); their sources, and the up to three of the next block that share the
@@ -222,20 +226,23 @@ int seam(const float* tX, const float* tY, const float* tZ, float* tW, const flo
       for (int a = 0; a <= DIM && c1 > c0; a++)
         PRBF_CUDA(cudaMemcpyAsync(S.src[a].get() + c0, sh[a] + c0, sizeof(float) * (c1 - c0), cudaMemcpyHostToDevice,
                                   S.s));
-      PRBF_CUDA(cudaEventRecord(S.in[p], S.s));
-      PRBF_CUDA(cudaStreamWaitEvent(S.k, S.in[p], 0));
-      k_seam<DIM><<<b1 - b0, kSlots, 0, S.k>>>(S.off.get(), S.t[0].get(), S.t[1].get(),
-                                               DIM == 3 ? S.t[2].get() : nullptr, tw_dev, c2, norm, S.src[0].get(),
-                                               S.src[1].get(), DIM == 3 ? S.src[2].get() : nullptr, S.src[DIM].get(),
-                                               S.err.get(), b0);
+      if (parts > 1) {
+        PRBF_CUDA(cudaEventRecord(S.in[p], S.s));
+        PRBF_CUDA(cudaStreamWaitEvent(S.k, S.in[p], 0));
+      }
+      k_seam<DIM><<<b1 - b0, kSlots, 0, ks>>>(S.off.get(), S.t[0].get(), S.t[1].get(),
+                                              DIM == 3 ? S.t[2].get() : nullptr, tw_dev, c2, norm, S.src[0].get(),
+                                              S.src[1].get(), DIM == 3 ? S.src[2].get() : nullptr, S.src[DIM].get(),
+                                              S.err.get(), b0);
       PRBF_CHECK_LAUNCH();
       c0 = std::max(c0, c1);
       b0 = b1;
     }
     unsigned herr = 0;
-    PRBF_CUDA(cudaMemcpyAsync(tW, tw_dev, sizeof(float) * nt, cudaMemcpyDeviceToHost, S.k));
-    PRBF_CUDA(cudaMemcpyAsync(&herr, S.err.get(), sizeof(unsigned), cudaMemcpyDeviceToHost, S.k));
-    PRBF_CUDA(cudaStreamSynchronize(S.k));
+    PRBF_CUDA(cudaMemcpyAsync(tW, tw_dev, sizeof(float) * nt, cudaMemcpyDeviceToHost, ks));
+    PRBF_CUDA(cudaMemcpyAsync(&herr, S.err.get(), sizeof(unsigned), cudaMemcpyDeviceToHost, ks));
+    PRBF_CUDA(cudaStreamSynchronize(ks));
+    drain.armed = false;  // (the kernels' stream has waited for every copy)
     if (herr) return PRBF_ERR_TIMEOUT;
     return PRBF_OK;
   } catch (const Error& e) {
