@@ -25,6 +25,8 @@
 // or (FP64, on request) factored by LU with partial pivoting.
 #include <algorithm>
 #include <cmath>
+#include <mutex>
+#include <set>
 #include <vector>
 
 #include "rasm.h"
@@ -1997,6 +1999,22 @@ void rasm_buffer_lists(const PointSet& P, int* counts_dev, const long long* boff
 }
 
 namespace {
+// A kernel's dynamic shared memory limit belongs to the function, so to every context of the
+// process: it is set once per device, to the most that the checks let through. (Set to each
+// plan's own size, a context with small blocks took the launches of another one's large blocks
+// away between their set-up and their use.)
+constexpr size_t kApplySmem = 220 * 1024, kAsmSmem = 200 * 1024;
+void allow_smem(const void* f, size_t bytes) {
+  static std::mutex m;
+  static std::set<std::pair<int, const void*>> done;
+  int dev = 0;
+  PRBF_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(m);
+  if (done.count({dev, f})) return;
+  PRBF_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  done.insert({dev, f});
+}
+
 // The LU fallback's blocks (cells, any order): K assembled unshifted into their own
 // storage, factored by k_lu_fp64; a zero pivot is the reference's PETSc LU failure.
 void lu_build(RasmPlan& R, const BlockGeom& G, const std::vector<int>& hcnt, std::vector<int> cells, Workspace& ws,
@@ -2121,11 +2139,11 @@ void rasm_factor(RasmPlan& R, const BlockGeom& G, const std::vector<int>& hcnt, 
   // FP32 assembly: the largest block's split coordinates in shared memory
   const size_t asm_smem = fp32 ? sizeof(float2) * (size_t)G.dim * std::max(R.max_nb, 1) : 0;
   if (fp32) {
-    if (asm_smem > 200 * 1024) throw Error(PRBF_ERR_CAPACITY, "subdomain larger than the assembly's shared memory");
-    PRBF_CUDA(cudaFuncSetAttribute(k_assemble<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)asm_smem));
-    PRBF_CUDA(cudaFuncSetAttribute(k_chol_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chol_tc_smem()));
+    if (asm_smem > kAsmSmem) throw Error(PRBF_ERR_CAPACITY, "subdomain larger than the assembly's shared memory");
+    allow_smem((const void*)k_assemble<float>, kAsmSmem);
+    allow_smem((const void*)k_chol_tc, chol_tc_smem());
   } else
-    PRBF_CUDA(cudaFuncSetAttribute(k_chol_fp64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem((const void*)k_chol_fp64, smem);
   R.nfallback = 0;
   R.retried.clear();
   R.nlu = 0;
@@ -2286,21 +2304,24 @@ void apply_tri_nv(const RasmPlan& R, const T* Lp, const int* cs, const double* r
 template <class T>
 void set_tri_smem(const RasmPlan& R) {
   for (int nv = 1; nv <= std::max(1, std::min(4, R.max_nv)); nv++) {
-    size_t sm;
-    const void* f;
     if constexpr (std::is_same<T, float>::value) {
-      sm = (size_t)kTrwWarps * nv * trw_ldy(R) * sizeof(float);
-      f = nv == 1 ? (const void*)k_apply_trw<1>
-                  : nv == 2 ? (const void*)k_apply_trw<2> : nv == 3 ? (const void*)k_apply_trw<3> : (const void*)k_apply_trw<4>;
+      if ((size_t)kTrwWarps * nv * trw_ldy(R) * sizeof(float) > kApplySmem)
+        throw Error(PRBF_ERR_CAPACITY, "subdomain larger than the apply kernel's shared memory");
+      allow_smem(nv == 1   ? (const void*)k_apply_trw<1>
+                 : nv == 2 ? (const void*)k_apply_trw<2>
+                 : nv == 3 ? (const void*)k_apply_trw<3>
+                           : (const void*)k_apply_trw<4>,
+                 kApplySmem);
     } else {
-      sm = (size_t)nv * std::max(R.max_nb, 1) * sizeof(T) + sizeof(T) * 32 * 33;
-      f = nv == 1 ? (const void*)k_apply_tri64<1>
-                  : nv == 2 ? (const void*)k_apply_tri64<2>
-                            : nv == 3 ? (const void*)k_apply_tri64<3> : (const void*)k_apply_tri64<4>;
+      constexpr size_t tri = sizeof(T) * 32 * 33;  // the kernel's own array
+      if ((size_t)nv * std::max(R.max_nb, 1) * sizeof(T) + tri > kApplySmem)
+        throw Error(PRBF_ERR_CAPACITY, "subdomain larger than the apply kernel's shared memory");
+      allow_smem(nv == 1   ? (const void*)k_apply_tri64<1>
+                 : nv == 2 ? (const void*)k_apply_tri64<2>
+                 : nv == 3 ? (const void*)k_apply_tri64<3>
+                           : (const void*)k_apply_tri64<4>,
+                 kApplySmem - tri);
     }
-    if (sm > 220 * 1024) throw Error(PRBF_ERR_CAPACITY, "subdomain larger than the apply kernel's shared memory");
-    PRBF_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(std::is_same<T, float>::value ? sm : sm - sizeof(T) * 32 * 33)));
   }
 }
 }  // namespace
@@ -2346,8 +2367,8 @@ void rasm_apply(const RasmPlan& R, const int* cs, const double* r, double* out, 
 void rasm_set_apply_smem(const RasmPlan& R) {
   if (R.nlu) {
     const size_t sm = (size_t)std::max(1, std::min(4, R.max_nv)) * std::max(R.max_nb, 1) * sizeof(double);
-    if (sm > 220 * 1024) throw Error(PRBF_ERR_CAPACITY, "subdomain larger than the LU apply's shared memory");
-    PRBF_CUDA(cudaFuncSetAttribute(k_apply_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (sm > kApplySmem) throw Error(PRBF_ERR_CAPACITY, "subdomain larger than the LU apply's shared memory");
+    allow_smem((const void*)k_apply_lu, kApplySmem);
   }
   if (R.factor) {
     if (R.fp32)
@@ -2355,9 +2376,9 @@ void rasm_set_apply_smem(const RasmPlan& R) {
     else
       set_tri_smem<double>(R);
   } else {
-    size_t sm = (size_t)std::max(R.max_nb, 1) * sizeof(float);
-    if (sm > 220 * 1024) throw Error(PRBF_ERR_CAPACITY, "subdomain larger than the apply kernel's shared memory");
-    PRBF_CUDA(cudaFuncSetAttribute(k_apply<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if ((size_t)std::max(R.max_nb, 1) * sizeof(float) > kApplySmem)
+      throw Error(PRBF_ERR_CAPACITY, "subdomain larger than the apply kernel's shared memory");
+    allow_smem((const void*)k_apply<float>, kApplySmem);
   }
 }
 
