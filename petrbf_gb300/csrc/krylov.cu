@@ -429,31 +429,38 @@ void Krylov::iteration(const Operator& op, cudaStream_t s, cudaGraphConditionalH
   PRBF_CHECK_LAUNCH();
 }
 
+// The iteration is captured into a graph of its own, which becomes a child of the while node's
+// body once the capture has succeeded: a launch that fails in it then leaves behind a captured
+// graph like any other, not a while node with half a body to be destroyed.
 void Krylov::build_graph(const Operator& op, cudaStream_t s) {
   reset_graph();
   PRBF_CUDA(cudaGraphCreate(&graph, 0));
   cudaGraphConditionalHandle cond;
   PRBF_CUDA(cudaGraphConditionalHandleCreate(&cond, graph, 1, cudaGraphCondAssignDefault));
+  struct Captured {
+    cudaGraph_t g = nullptr;
+    ~Captured() {
+      if (g) cudaGraphDestroy(g);
+    }
+  } it;
+  PRBF_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
+  try {
+    iteration(op, s, cond, 1);
+  } catch (...) {
+    cudaStreamEndCapture(s, &it.g);  // (null when the capture was invalidated)
+    cudaGetLastError();
+    reset_graph();
+    throw;
+  }
+  PRBF_CUDA(cudaStreamEndCapture(s, &it.g));
   cudaGraphNodeParams cp = {};
   cp.type = cudaGraphNodeTypeConditional;
   cp.conditional.handle = cond;
   cp.conditional.type = cudaGraphCondTypeWhile;
   cp.conditional.size = 1;
-  cudaGraphNode_t node;
+  cudaGraphNode_t node, child;
   PRBF_CUDA(cudaGraphAddNode(&node, graph, nullptr, nullptr, 0, &cp));
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-  PRBF_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-  try {
-    iteration(op, s, cond, 1);
-  } catch (...) {
-    cudaGraph_t dummy = nullptr;
-    cudaStreamEndCapture(s, &dummy);
-    cudaGetLastError();
-    graph_op = nullptr;
-    throw;
-  }
-  cudaGraph_t captured;
-  PRBF_CUDA(cudaStreamEndCapture(s, &captured));
+  PRBF_CUDA(cudaGraphAddChildGraphNode(&child, cp.conditional.phGraph_out[0], nullptr, 0, it.g));
   PRBF_CUDA(cudaGraphInstantiate(&exec, graph, 0));
   graph_op = &op;
 }
