@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <mutex>
 
 #include "device.h"
 #include "gauss_common.cuh"
@@ -1411,12 +1412,15 @@ __global__ void k_trunc_count(Grid g, const int* __restrict__ cs_t, const double
   }
 }
 
-bool g_tab_ready[64] = {false};
-
+// Once per device; contexts of several threads may ask at the same time (the flag, and the
+// host copies that one of them would still be filling).
 void upload_table(cudaStream_t s) {
+  static std::mutex m;
+  static bool ready[64] = {false};
   int dev = 0;
   PRBF_CUDA(cudaGetDevice(&dev));
-  if (dev < 64 && g_tab_ready[dev]) return;
+  std::lock_guard<std::mutex> lk(m);
+  if (dev < 64 && ready[dev]) return;
   // Large table: c_i = monomial coefficients of the cubic through (r_k, e^(L r_k)) at the
   // Chebyshev nodes r_k = cos((2k+1) pi / 8) / 2 (Newton divided differences, then
   // expanded), in long double; small table: c_i = L^i / i!. Then T[j] = 2^(-j/n) and the
@@ -1458,7 +1462,7 @@ void upload_table(cudaStream_t s) {
   PRBF_CUDA(cudaMemcpyToSymbolAsync(d_tab_big, h2, sizeof(h2), 0, cudaMemcpyHostToDevice, s));
   PRBF_CUDA(cudaMemcpyToSymbolAsync(d_tab_small, h3, sizeof(h3), 0, cudaMemcpyHostToDevice, s));
   PRBF_CUDA(cudaStreamSynchronize(s));
-  if (dev < 64) g_tab_ready[dev] = true;
+  if (dev < 64) ready[dev] = true;
 }
 
 template <int DIM, bool F32, int NV>
