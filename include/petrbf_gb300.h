@@ -133,6 +133,15 @@ const char* prbf_status_string(int status);
  * their destruction (:296-307) -- kept across calls with its device memory and one stream. */
 int prbf_ctx_create(const prbf_params* p, prbf_ctx** out);
 int prbf_ctx_destroy(prbf_ctx* ctx);
+/* Device memory kept between calls (no reference counterpart). Buffers of up to 256 MB that a
+ * call or a destroyed context no longer needs stay with the process, at most 2 GB per device,
+ * and serve later calls and contexts; the oldest make room for newer ones. They go back to the
+ * driver when an allocation of this library fails, when 16 contexts have come and gone without
+ * using them, and on request: another allocator of the process sees them as taken until then.
+ * prbf_memory_kept returns the bytes kept on a device (0 for one never used),
+ * prbf_memory_release gives them back; any thread may call either at any time. */
+long long prbf_memory_kept(int device);
+int prbf_memory_release(int device);
 /* Last error message of this context (valid until the next call on it; no reference
  * counterpart: CHKERRQ prints and returns). */
 const char* prbf_last_error(const prbf_ctx* ctx);

@@ -74,6 +74,8 @@ SIGNATURES = {
     "prbf_status_string": (ctypes.c_char_p, [ctypes.c_int]),
     "prbf_ctx_create": (ctypes.c_int, [ctypes.POINTER(Params), ctypes.POINTER(ctypes.c_void_p)]),
     "prbf_ctx_destroy": (ctypes.c_int, [ctypes.c_void_p]),
+    "prbf_memory_kept": (ctypes.c_longlong, [ctypes.c_int]),
+    "prbf_memory_release": (ctypes.c_int, [ctypes.c_int]),
     "prbf_last_error": (ctypes.c_char_p, [ctypes.c_void_p]),
     "prbf_ctx_stream": (ctypes.c_void_p, [ctypes.c_void_p]),
     "prbf_ctx_synchronize": (ctypes.c_int, [ctypes.c_void_p]),

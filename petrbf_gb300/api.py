@@ -208,6 +208,16 @@ class Context:
         return w
 
 
+def memory_kept(device=0):
+    """Bytes of device memory that the library keeps for later calls."""
+    return int(N.lib().prbf_memory_kept(int(device)))
+
+
+def release_memory(device=0):
+    """Gives the device memory kept for later calls back to the driver."""
+    N.lib().prbf_memory_release(int(device))
+
+
 def batch_interpolate(problems, dim=2, rtol=1e-13, restart=30, max_it=1000, pc="asm", device=0,
                       precision="fp64", block_fallback="shift"):
     """Solves many independent problems together. problems: sequence of dicts with keys x,

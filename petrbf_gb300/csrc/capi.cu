@@ -213,6 +213,13 @@ int prbf_ctx_destroy(prbf_ctx* ctx) {
   return PRBF_OK;
 }
 
+long long prbf_memory_kept(int device) { return (long long)dev_pool_kept(device); }
+
+int prbf_memory_release(int device) {
+  dev_pool_trim(device);
+  return PRBF_OK;
+}
+
 const char* prbf_last_error(const prbf_ctx* ctx) { return ctx ? ctx->c.last_error.c_str() : "null context"; }
 
 void* prbf_ctx_stream(prbf_ctx* ctx) { return ctx ? (void*)ctx->c.stream : nullptr; }

@@ -27,8 +27,11 @@ cudaError_t dev_alloc(void** p, size_t bytes);
 void dev_free(void* p);
 // The stream is idle and about to be destroyed: its blocks may serve others.
 void dev_pool_stream_done(int device, cudaStream_t s);
-// Gives the current device's kept blocks back to the driver.
-void dev_pool_trim();
+// Gives a device's kept blocks back to the driver; their bytes.
+void dev_pool_trim(int device);
+size_t dev_pool_kept(int device);
+// Free memory of the current device, kept blocks included.
+size_t dev_mem_free();
 
 // Owning device buffer, grow-only.
 template <class T>

@@ -7,10 +7,14 @@
 // context's, set for the length of a call, StreamScope) and serves the same stream again at once,
 // ordered behind that work; other streams get it once its own is known to be idle
 // (dev_pool_stream_done, when the context is destroyed). Calls outside of any context allocate and
-// free as before. Bounded: blocks up to kMaxBlock, kMaxCached bytes per device; given back when an
-// allocation fails, and when 16 contexts have come and gone without a use.
+// free as before. Bounded: blocks up to kMaxBlock, kMaxCached bytes per device, beyond which the
+// blocks that have lain longest make room. Given back when an allocation fails, when 16 contexts
+// have come and gone without a use, and on request (prbf_memory_release). What is kept counts as
+// free memory where a size is chosen by it (dev_mem_free), so that no choice depends on the calls
+// that came before.
 #include <map>
 #include <mutex>
+#include <new>
 #include <unordered_map>
 #include <vector>
 
@@ -27,14 +31,16 @@ thread_local bool t_on = false, t_idle = false;
 
 struct Free {
   void* p;
-  cudaStream_t stream;  // may still have work on the block; null: idle
-  unsigned long long since;
+  cudaStream_t stream;       // may still have work on the block; null: idle
+  unsigned long long since;  // contexts destroyed when it was freed
+  unsigned long long turn;   // frees before it
 };
 
 struct DevicePool {
   std::multimap<size_t, Free> free;
   size_t cached = 0;
   unsigned long long epoch = 0;  // contexts destroyed
+  unsigned long long turn = 0;   // blocks freed
 };
 
 struct Pool {
@@ -75,6 +81,18 @@ std::vector<void*> take(DevicePool& D, bool all) {
   return out;
 }
 
+// Takes out the blocks that have lain longest until a block of cls bytes fits beside the rest.
+void make_room(DevicePool& D, size_t cls, std::vector<void*>& out) {
+  while (D.cached + cls > kMaxCached) {
+    auto old = D.free.begin();
+    for (auto it = D.free.begin(); it != D.free.end(); ++it)
+      if (it->second.turn < old->second.turn) old = it;
+    out.push_back(old->second.p);
+    D.cached -= old->first;
+    D.free.erase(old);
+  }
+}
+
 }  // namespace
 
 StreamScope::StreamScope(cudaStream_t s, bool idle) : stream(t_stream), on(t_on), was_idle(t_idle) {
@@ -95,7 +113,7 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaErrorMemoryAllocation) return e;
     cudaGetLastError();
-    dev_pool_trim();
+    dev_pool_trim(current_device());
     return cudaMalloc(p, bytes);
   }
   Pool& P = pool();
@@ -121,7 +139,7 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, cls);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    dev_pool_trim();
+    dev_pool_trim(d);
     return cudaMalloc(p, bytes);  // (as asked for; not the pool's)
   }
   if (e == cudaSuccess) {
@@ -133,21 +151,25 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
 
 void dev_free(void* p) {
   Pool& P = pool();
-  {
+  std::vector<void*> out;  // (cudaFree waits for work on what it frees, whatever its stream)
+  try {
     std::lock_guard<std::mutex> lk(P.m);
     auto it = P.used.find(p);
     if (it != P.used.end()) {
       const auto [d, cls] = it->second;
       P.used.erase(it);
-      DevicePool& D = P.dev[d];
-      if (t_on && D.cached + cls <= kMaxCached) {
-        D.free.insert({cls, Free{p, t_idle ? nullptr : t_stream, D.epoch}});
+      if (t_on) {
+        DevicePool& D = P.dev[d];
+        make_room(D, cls, out);
+        D.free.insert({cls, Free{p, t_idle ? nullptr : t_stream, D.epoch, D.turn++}});
         D.cached += cls;
-        return;
+        p = nullptr;
       }
     }
+  } catch (const std::bad_alloc&) {  // (buffers are freed by destructors)
   }
-  cudaFree(p);
+  if (p) cudaFree(p);
+  for (void* q : out) cudaFree(q);
 }
 
 void dev_pool_stream_done(int device, cudaStream_t s) {
@@ -164,15 +186,26 @@ void dev_pool_stream_done(int device, cudaStream_t s) {
   for (void* p : old) cudaFree(p);
 }
 
-void dev_pool_trim() {
+void dev_pool_trim(int device) {
   Pool& P = pool();
   std::vector<void*> all;
   {
     std::lock_guard<std::mutex> lk(P.m);
-    int d = 0;
-    if (cudaGetDevice(&d) == cudaSuccess) all = take(P.dev[d], true);
+    all = take(P.dev[device], true);
   }
   for (void* p : all) cudaFree(p);
+}
+
+size_t dev_pool_kept(int device) {
+  Pool& P = pool();
+  std::lock_guard<std::mutex> lk(P.m);
+  return P.dev[device].cached;
+}
+
+size_t dev_mem_free() {
+  size_t free_b = 0, total_b = 0;
+  PRBF_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  return free_b + dev_pool_kept(current_device());
 }
 
 }  // namespace prbf

@@ -1744,8 +1744,7 @@ void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& sr
     const int W = 2 * g.nb_trunc + 1;
     const int K = g.dim == 2 ? (W * W - 1) / 2 : (W * W * W - 1) / 2;
     const long long pstride = ((long long)src.n + 8 + 31) / 32 * 32;
-    size_t free_b = 0, total_b = 0;
-    PRBF_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    const size_t free_b = dev_mem_free();
     const int nvs = std::max(1, std::min(4, plan.sym_nv));
     const int sets = plan.fx_ready && hmax > kFxSymTile ? 2 : 1;
     const double bytes = (double)K * sets * nvs * pstride * sizeof(double) + (double)(src.n + 8) * 8;
@@ -1792,8 +1791,7 @@ bool gauss_plan_sym_batch(GaussPlan& plan, const std::vector<Grid>& grids, const
   std::stable_sort(its.begin(), its.end(),
                    [&](const int2& a, const int2& b) { return hcs[a.x + 1] - hcs[a.x] > hcs[b.x + 1] - hcs[b.x]; });
   const long long pstride = ((long long)src.n + 8 + 31) / 32 * 32;
-  size_t free_b = 0, total_b = 0;
-  PRBF_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  const size_t free_b = dev_mem_free();
   if ((double)K * sets * pstride * sizeof(double) + (double)(src.n + 8) * 8 > 0.125 * (double)free_b) return false;
   plan.sym_K = K;
   plan.sym_sets = sets;

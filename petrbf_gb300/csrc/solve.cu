@@ -117,8 +117,7 @@ static void interpolate(Ctx& c, int n, const double* x, const double* y, const d
   const bool mixed = p.precision == PRBF_PREC_MIXED;
   gauss_plan_dev(S.plan, S.pts.view(), S.pts.view(), c.err.get(), c.ws, c.stream,
                  PLAN_COUNTS | FORM_F64 | (mixed ? FORM_F32 : 0));
-  size_t free_b = 0, total_b = 0;
-  PRBF_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  const size_t free_b = dev_mem_free();
   double budget = std::min(16.0e9, 0.25 * (double)free_b);
   // FP32 blocks: S_c (one GEMV per apply) in 2D; in 3D the blocks are too ill-conditioned
   // for an explicit FP32 inverse, so the FP32 factor is kept and applied by substitution
@@ -399,8 +398,7 @@ int prbf_pc_setup(prbf_ctx* ctx, int precision) {
     if (precision != PRBF_PREC_FP64 && precision != PRBF_PREC_MIXED) throw Error(PRBF_ERR_ARG, "bad precision");
     if (!c.solve) c.solve = new SolveState();
     c.solve->pc_ready = false;
-    size_t free_b = 0, total_b = 0;
-    PRBF_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    const size_t free_b = dev_mem_free();
     const bool fp32 = precision == PRBF_PREC_MIXED;
     c.solve->pc.lu_fallback = c.p.block_fallback == PRBF_FALLBACK_LU;
     rasm_build(c.solve->pc, c.mv_pts, fp32, c.ws, c.err.get(), c.stream, std::min(16.0e9, 0.25 * (double)free_b),
