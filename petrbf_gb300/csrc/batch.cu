@@ -310,7 +310,7 @@ void batch_interpolate(Ctx& c, int nprob, const prbf_problem* probs, int* its_ou
   PRBF_CUDA(cudaMemcpyAsync(B.plan.cprob.get(), B.cprob.get(), sizeof(int) * NC, cudaMemcpyDeviceToDevice, c.stream));
   gauss_plan_forms_batch(B.plan, hgrids,
                          PointsView{N, B.x.get(), B.y.get(), dim == 3 ? B.z.get() : nullptr, B.cs.get()},
-                         FORM_F64 | (mixed ? FORM_F32 : 0), c.stream);
+                         mixed ? FORM_F32 | form64_of_refinement(dim) : FORM_F64, c.stream);
 
   // ---- pass 2: buffer lists into the global block arrays, then one batched factorisation
   std::vector<long long> hb((size_t)NC + 1);

@@ -135,7 +135,6 @@ struct GaussPlan {
   // targets' where they are another point set
   bool fx_ready = false;
   bool fx_self = true;
-  bool pipe64 = false;  // FP64 sums by the FP64 pipe's kernels all the same (see solve.cu)
   int fx_ncs = 0;       // entries of the cell starts
   DevBuf<uint2> fxs[3], fxt[3];
   // FP64 matvec with each exponential used for both rows (targets == sources, every cell
@@ -157,8 +156,15 @@ struct GaussPlan {
 // What a plan is used for: the FP32 products, the FP64 products (neither for a plan used only
 // for its sizes), the truncation-set sizes (trunc_cnt, pairs, max_trunc; zero when not asked
 // for -- a single evaluation has no use for them, and they are 200 us of 1.7 ms at 5x10^5
-// sources and 3x10^5 targets).
-enum : int { FORM_F32 = 1, FORM_F64 = 2, PLAN_COUNTS = 4 };
+// sources and 3x10^5 targets). FORM_PIPE64: FP64 products whose exponentials stay on the FP64
+// pipe (form64_of_refinement).
+enum : int { FORM_F32 = 1, FORM_F64 = 2, PLAN_COUNTS = 4, FORM_PIPE64 = 8 };
+// The FP64 products of a mixed-precision refinement, a single solve's or a batch's. 3D keeps the
+// FP64 pipe's kernels: it ends at the rounding floor of the residual (2e-15 of |f| on 56^3
+// points, cond(A) above 1e7), where any other rounding of the sums moves single weights by up to
+// 6e-8 of their root mean square, no closer to the solution (fixed-point sums: 483 against 612 ms
+// for those 56^3 points and three right-hand sides). 2D weights move by 4e-10 at most.
+inline int form64_of_refinement(int dim) { return dim == 3 ? FORM_PIPE64 : FORM_F64; }
 // Builds the work list, the truncation-set sizes and the point data as asked for.
 void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& src,
                     unsigned* err, Workspace& ws, cudaStream_t s, int forms = FORM_F32 | FORM_F64 | PLAN_COUNTS);

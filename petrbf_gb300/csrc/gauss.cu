@@ -1701,14 +1701,17 @@ void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& sr
   plan.sym_ready = false;
   plan.sym_nitems = 0;
   plan.sym_ncs = 0;
-  if (!(forms & (FORM_F32 | FORM_F64))) return;
+  const bool f64 = forms & (FORM_F64 | FORM_PIPE64);
+  if (!(forms & FORM_F32) && !f64) return;
   const bool self = tgt.x == src.x && tgt.n == src.n;
   if (f32_grid_ok(g) && src.n > 0) {
     const bool f32 = forms & FORM_F32, fx = (forms & FORM_F64) && fx_grid_ok(g);
-    const PointForms o = alloc_forms(plan, g.dim, src.n, f32, fx, s);
-    k_point_forms<<<ceil_div(g.ncell, 8), 256, 0, s>>>(g, nullptr, nullptr, g.ncell, src.cell_start, src.x, src.y,
-                                                       src.z, o);
-    PRBF_CHECK_LAUNCH();
+    if (f32 || fx) {
+      const PointForms o = alloc_forms(plan, g.dim, src.n, f32, fx, s);
+      k_point_forms<<<ceil_div(g.ncell, 8), 256, 0, s>>>(g, nullptr, nullptr, g.ncell, src.cell_start, src.x, src.y,
+                                                         src.z, o);
+      PRBF_CHECK_LAUNCH();
+    }
     if (fx) {
       gauss_fx_upload_tables(s);
       plan.fx_self = self;
@@ -1727,7 +1730,7 @@ void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& sr
   }
   // (the fixed-point form's symmetric sum is 2D, one vector: with more vectors, or 3D's wider
   // windows, its one-sided sum is bound by the same multiply-adds and writes no slots)
-  if (!(forms & FORM_F64) || (plan.fx_ready && (g.dim == 3 || plan.sym_nv > 1))) return;
+  if (!f64 || (plan.fx_ready && (g.dim == 3 || plan.sym_nv > 1))) return;
   // symmetric FP64 matvec: the same point set on both sides, every cell within one item
   // (<= kTileT points), 2 nb + 1 mask bits per axis, at most kSymMaxK partial slots per
   // point and vector (each product writes and gathers them: the 7 x 7 x 7 window of a 3D
@@ -1828,6 +1831,7 @@ void gauss_plan_forms_batch(GaussPlan& plan, const std::vector<Grid>& grids, con
     ncell += g.ncell;
   }
   const bool f32 = forms & FORM_F32;
+  if (!f32 && !fx) return;
   const PointForms o = alloc_forms(plan, grids[0].dim, src.n, f32, fx, s);
   k_point_forms<<<ceil_div(ncell, 8), 256, 0, s>>>(plan.g, plan.grids.get(), plan.cprob.get(), ncell, src.cell_start,
                                                    src.x, src.y, src.z, o);
@@ -1856,7 +1860,7 @@ void gauss_sum_dev(const GaussPlan& P, const PointsView& t, const PointsView& s,
     }
     return;
   }
-  if (!fp32 && P.fx_ready && !P.pipe64) {
+  if (!fp32 && P.fx_ready) {
     gauss_fx_sum(P, t, s, gv, w, err, skip, nv, vstride, left, st);
     return;
   }

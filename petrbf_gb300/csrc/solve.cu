@@ -116,7 +116,7 @@ static void interpolate(Ctx& c, int n, const double* x, const double* y, const d
   S.plan.sym_nv = std::min(4, nrhs);  // right-hand sides summed together by the symmetric form
   const bool mixed = p.precision == PRBF_PREC_MIXED;
   gauss_plan_dev(S.plan, S.pts.view(), S.pts.view(), c.err.get(), c.ws, c.stream,
-                 PLAN_COUNTS | FORM_F64 | (mixed ? FORM_F32 : 0));
+                 PLAN_COUNTS | (mixed ? FORM_F32 | form64_of_refinement(dim) : FORM_F64));
   const size_t free_b = dev_mem_free();
   double budget = std::min(16.0e9, 0.25 * (double)free_b);
   // FP32 blocks: S_c (one GEMV per apply) in 2D; in 3D the blocks are too ill-conditioned
@@ -214,12 +214,6 @@ static void interpolate(Ctx& c, int n, const double* x, const double* y, const d
       st.guess_rel_resid = gres;
     }
   };
-  // 3D refinement keeps its FP64 residuals on the FP64 pipe's kernels: it ends at the rounding
-  // floor of the residual (2e-15 of |f| on 56^3 points, cond(A) above 1e7), where any other
-  // rounding of the sums moves single weights by up to 6e-8 of their root mean square, no
-  // closer to the solution (fixed-point sums: 483 against 612 ms for those 56^3 points and
-  // three right-hand sides). 2D weights move by 4e-10 at most.
-  S.plan.pipe64 = mixed && dim == 3;
   if (!mixed) {
     plain_solve(use_guess);
   } else {
@@ -317,7 +311,8 @@ static void interpolate(Ctx& c, int n, const double* x, const double* y, const d
     if (stalled) {
       // FP64 blocks and FP64 GMRES from zero for every right-hand side (the inner
       // iterations spent so far stay counted)
-      S.plan.pipe64 = false;
+      if (form64_of_refinement(dim) != FORM_F64)
+        gauss_plan_dev(S.plan, S.pts.view(), S.pts.view(), c.err.get(), c.ws, c.stream, FORM_F64);
       S.kry.reset_graph();
       rasm_build(S.rasm, S.pts, false, c.ws, c.err.get(), c.stream, budget, false, p.pc_type == PRBF_PC_ASM);
       rasm_set_apply_smem(S.rasm);
