@@ -5,6 +5,7 @@
 #include <cstring>
 
 #include "context.h"
+#include "gauss_fx.cuh"
 
 namespace prbf {
 
@@ -40,7 +41,7 @@ Grid make_grid(int dim, const double* b, double sigma, int nsigma_box, int sigma
   g.ncell = g.nx * g.ny * g.nz;
   g.trunc_len = sigma_trunc * sigma / 2 + kEpsf;
   g.buffer_len = sigma_buffer * sigma / 2 + kEpsf;
-  g.norm = 1.0 / (2 * 3.141592653589793 * sigma * sigma);
+  g.norm = gauss_norm(sigma);
   return g;
 }
 

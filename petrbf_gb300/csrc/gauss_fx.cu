@@ -50,6 +50,7 @@ constexpr int kCons = SYM ? 8 : 11;
 template <bool SYM>
 constexpr int kFxThreads = 32 * (kCons<SYM> + (SYM ? 2 : 1));
 constexpr int kResident = 2 * 152;  // CTAs resident on the GPU
+constexpr int kJoin = 2;            // buffers from one joining of the lanes' sums to the next
 
 __device__ uint2 d_fx_t1[kFxTab], d_fx_t2[kFxTab];
 
@@ -79,7 +80,9 @@ struct LayoutX {
   // per consumer warp and target: coordinates and (SYM) weight and box-test word
   static constexpr int TW = DIM + (SYM ? 2 : 0);
   static constexpr size_t tgt = align16(tab2 + 8 * (size_t)kFxTab);
-  static constexpr size_t total = align16(tgt + 8 * (size_t)TW * C::TT);
+  // one-sided: a target's running totals, each with what its additions rounded away
+  static constexpr size_t tot = align16(tgt + 8 * (size_t)TW * C::TT);
+  static constexpr size_t total = align16(tot + (SYM ? 0 : 16 * (size_t)NV * C::TT));
 };
 
 // exp of a pair: coordinates (l, h) of target and source
@@ -96,7 +99,7 @@ __device__ __forceinline__ double fx_pair(const uint2 (&t)[DIM], const uint2 (&s
 // The lanes' sums of N <= 8 values over the warp, by a butterfly that halves the values each
 // lane carries while there are two or more (N = 8: 9 FP64 adds a lane instead of 8 x 5). Lane l
 // returns the total of value *which (-1: of none). Every value is added up in the same order
-// whatever N.
+// whatever N: neighbouring lanes first.
 template <int N>
 __device__ __forceinline__ double fx_scatter_sum(const double (&a)[N], int lane, int& which) {
   constexpr unsigned F = 0xffffffffu;
@@ -105,7 +108,7 @@ __device__ __forceinline__ double fx_scatter_sum(const double (&a)[N], int lane,
 #pragma unroll
   for (int i = 0; i < P; i++) k[i] = i < N ? a[i] : 0.0;
   which = 0;
-  int bit = 16;
+  int bit = 1;
 #pragma unroll
   for (int h = P / 2; h >= 1; h /= 2) {
     const bool up = lane & bit;
@@ -115,11 +118,10 @@ __device__ __forceinline__ double fx_scatter_sum(const double (&a)[N], int lane,
       k[i] = mine + __shfl_xor_sync(F, other, bit);
     }
     which += up ? h : 0;
-    bit >>= 1;
+    bit <<= 1;
   }
-  for (; bit > 0; bit >>= 1) k[0] += __shfl_xor_sync(F, k[0], bit);
-  const int low = 32 / P - 1;  // lanes that differ in these bits hold the same total
-  if ((lane & low) != 0 || which >= N) which = -1;
+  for (; bit < 32; bit <<= 1) k[0] += __shfl_xor_sync(F, k[0], bit);
+  if (lane >= P || which >= N) which = -1;  // (lanes that differ in the other bits hold the same total)
   return k[0];
 }
 
@@ -167,7 +169,11 @@ __device__ __forceinline__ bool fx_consume(unsigned char* smem, FxShared& sh, co
     for (int k = 0; k < N; k++) acc[v][k] = 0.0;
   constexpr int TW = Lay::TW;
   uint2* tw = (uint2*)(smem + Lay::tgt) + wid * C::TG * TW;
+  double2* tot = (double2*)(smem + Lay::tot) + wid * C::TG * NV;
   if (lane < N) {
+    if constexpr (!SYM)
+#pragma unroll
+      for (int v = 0; v < NV; v++) tot[lane * NV + v] = make_double2(0.0, 0.0);
     tw[lane * TW] = a.tx[t + lane];
     tw[lane * TW + 1] = a.ty[t + lane];
     if constexpr (DIM == 3) tw[lane * TW + 2] = a.tz[t + lane];
@@ -177,20 +183,29 @@ __device__ __forceinline__ bool fx_consume(unsigned char* smem, FxShared& sh, co
     }
   }
   __syncwarp();
-  // after every buffer (one-sided form) the lanes' sums meet and join their target's running
-  // total: the partial sums stay short, as rounding grows with their length (a 3D target has
-  // some 10^4 sources)
-  double run[NV];
-  int which = -1;
-#pragma unroll
-  for (int v = 0; v < NV; v++) run[v] = 0.0;
+  // after every kJoin buffers (one-sided form) the lanes' sums meet and join their target's
+  // running total, which keeps what its additions round away: the lanes' partial sums stay short,
+  // as rounding grows with their length (a 3D target has some 10^4 sources), and the additions at
+  // the total's full size, one per join, cost nothing of it. (The totals lie in shared memory; in
+  // registers the 3D kernel spills, 18.0 against 17.8 ms on 96^3. With joins after 1, 2, 3, 4
+  // buffers the product took 18.2, 17.8, 17.7, 17.6 ms; three already lose on 40^3 points what the
+  // kept roundings gain.)
+  double sum[NV];
+  int which = -1, held = 0;
   auto join = [&]() {
     if constexpr (N > 0) {
 #pragma unroll
       for (int v = 0; v < NV; v++) {
-        run[v] += fx_scatter_sum<N>(acc[v], lane, which);
+        sum[v] = fx_scatter_sum<N>(acc[v], lane, which);
 #pragma unroll
         for (int k = 0; k < N; k++) acc[v][k] = 0.0;
+        if (!SYM && which >= 0) {
+          double2 q = tot[which * NV + v];
+          const double run = q.x + sum[v], d = run - q.x;
+          q.y += (q.x - (run - d)) + (sum[v] - d);
+          q.x = run;
+          tot[which * NV + v] = q;
+        }
       }
     }
   };
@@ -260,13 +275,27 @@ __device__ __forceinline__ bool fx_consume(unsigned char* smem, FxShared& sh, co
     if (lane == 0) mbar_arrive(&sh.empty[b]);
     ph ^= b;
     b ^= 1;
-    if (!SYM || last) join();
+    if constexpr (SYM) {
+      if (last) join();
+    } else {
+      if (last || ++held == kJoin) {
+        join();
+        held = 0;
+      }
+    }
     if (last) break;
   }
   if (N > 0 && which >= 0) {
 #pragma unroll
-    for (int v = 0; v < NV; v++) a.w[vm[v] * a.vs + t + which] = run[v] * norm;
+    for (int v = 0; v < NV; v++) {
+      if constexpr (!SYM) {  // (an infinite total leaves no number in what it rounded away)
+        const double2 q = tot[which * NV + v];
+        sum[v] = q.y == q.y ? q.x + q.y : q.x;
+      }
+      a.w[vm[v] * a.vs + t + which] = sum[v] * norm;
+    }
   }
+  if constexpr (!SYM) __syncwarp();  // the totals are read: the next pass may clear them
   return true;
 }
 

@@ -17,12 +17,15 @@
 //   2^(r / 2^54)  = 1 + r (c1 + c2 r) 2^-54,
 // u and t integers of 32 bits whose rounding errors e1 and e2 go into the last factor: with
 // V = u t (64 bits, one multiplication) and P = r (c1 + c2 r) + e1 + e2 the mantissa is
-// (V + V P 2^-54) 2^-10. Everything is truncated; the tables' e1 and e2 hold the mean of what
-// that drops, such that the zero exponent still gives exactly 1.
-// Against 64-bit-mantissa exponentials of 4x10^6 random arguments: mean error 2.0e-17, rms
-// 9.8e-17, largest 5.3e-16. (The 1024-entry table and cubic on the FP64 pipe, for exponents
-// below 1, 10 and 50, where the rounding of its exponent factor grows in: mean 1.1e-17,
-// 5.4e-17, 2.5e-16; rms 8.2e-17, 1.0e-16, 3.0e-16; largest 2.9e-16, 3.8e-16, 7.6e-16.)
+// (V + V P 2^-54) 2^-10. The shift of V and the product are centred by half a unit each, the
+// smaller truncations by e2, such that the zero exponent still gives exactly 1.
+// Against 64-bit-mantissa exponentials of 4x10^6 random arguments below 1, 10 and 50: mean error
+// -6.6e-18, -7.6e-18, -7.8e-18; rms 7.6e-17, 7.9e-17, 7.9e-17; largest 4.1e-16. (The 1024-entry
+// table and cubic on the FP64 pipe, where the rounding of its exponent factor, sigma's, grows in;
+// over five widths: mean up to 5.3e-17, 5.8e-16, 2.9e-15; rms 7.8e-17 to 1.0e-16, 9.9e-17 to
+// 6.7e-16, 3.2e-16 to 3.4e-15; largest 2.9e-16 to 3.6e-16, 3.8e-16 to 1.4e-15, 7.9e-16 to 6.1e-15.)
+// Keeping the bits that the shift drops (one 32 x 32 -> 64-bit product and two instructions more)
+// gives rms 6.1e-17 and largest 3.1e-16, and costs the 3D sum 5 %.
 #pragma once
 #include <cmath>
 
@@ -47,11 +50,11 @@ __host__ __device__ __forceinline__ unsigned fx_mulhi(unsigned a, unsigned b) {
 // 2^((B - kFxBias) 2^-54) as an FP64 number's bits, from B's words and the entries (u, e1) of
 // the bits 21..11 and (t, e2) of the bits 10..0 of its high one.
 __host__ __device__ __forceinline__ unsigned long long fx_pow2_bits(unsigned bh, unsigned r, uint2 p, uint2 q) {
-  // c1 = ln2 2^32, c2 = ln2^2 / 2 2^10
-  const unsigned c = fx_mulhi(r, 246u) + 2977044472u;
-  const unsigned P = fx_mulhi(r, c) + p.y + q.y;
-  const unsigned long long V = (unsigned long long)p.x * q.x;
-  const unsigned X = fx_mulhi((unsigned)(V >> 32), P);
+  // c1 = ln2 2^32, c2 = ln2^2 / 2 2^10; e's product with r c1 (up to 2^32) reaches three units
+  const unsigned e = p.y + q.y, c = fx_mulhi(r, 246u) + (2977044472u + (e >> 22));
+  const unsigned P = fx_mulhi(r, c) + e;
+  const unsigned long long V = (unsigned long long)p.x * q.x + 1024u;  // half a unit for each of
+  const unsigned X = fx_mulhi((unsigned)(V >> 32), P);                 // these two truncations
   // V's leading bit (62) lands on the exponent field's lowest
   return (V >> 10) + X + ((unsigned long long)((bh >> 2) & 0x3ff00000u) << 32);
 }
@@ -102,18 +105,31 @@ __host__ __device__ inline FxScale fx_scale(double sigma) {
   return FxScale{y * two58, 0.5 * y * res * two58};
 }
 
-// The tables, in long double. The truncations of fx_pow2_bits drop 4.7 units of 2^-54 on
-// average: e2 gets three of them, e1 two -- but e1[0] none, where P = 3 must still vanish in
-// the product with V's high word (2^30), so that a zero exponent gives exactly 1.
+// 1 / (2 pi sigma^2) rounded once (to within 2^-54 of its last place): the products and sums that
+// it is multiplied with carry less than the two units that rounding each of its operations would
+// put into every result alike.
+inline double gauss_norm(double sigma) {
+  const double plain = 1.0 / (2 * 3.141592653589793 * sigma * sigma);
+  if (!(sigma > 1e-100 && sigma < 1e100)) return plain;
+  const double p1 = 6.283185307179586, p2 = 2.4492935982947064e-16;  // 2 pi to 107 bits
+  const double s1 = sigma * sigma, s2 = std::fma(sigma, sigma, -s1);
+  const double q1 = s1 * p1, q2 = std::fma(s1, p1, -q1) + (s1 * p2 + s2 * p1);
+  const double n = 1.0 / q1;
+  return std::fma(n, std::fma(-n, q1, 1.0) - n * q2, n);
+}
+
+// The tables, in long double. The truncations in P drop one unit of 2^-54 on average, which e2
+// gets. A zero exponent gives exactly 1: u(0) is one less than 2^31 and P = 2^23 makes up for it,
+// V >> 10 = 2^52 - 2^21 + 1 and X = 2^21 - 1 (the entry of j1 = 0 is a unit low for that).
 inline void fx_tables(uint2* t1, uint2* t2) {
   const long double unit = 18014398509481984.0L, one = 2147483648.0L;  // 2^54, 2^31
   for (int j = 0; j < kFxTab; j++) {
-    const long double v = exp2l((long double)j / kFxTab) * one, u = floorl(v);
+    const long double v = exp2l((long double)j / kFxTab) * one, u = j ? floorl(v) : one - 1.0L;
     t1[j].x = (unsigned)u;
-    t1[j].y = (unsigned)llrintl((v - u) / u * unit) + (j ? 2u : 0u);
+    t1[j].y = j ? (unsigned)llrintl((v - u) / u * unit) : (1u << 23) - 1u;
     const long double x = expm1l((long double)j / 4194304.0L * logl(2.0L)) * one, t = floorl(x);
     t2[j].x = 2147483648u + (unsigned)t;
-    t2[j].y = (unsigned)llrintl((x - t) / (one + t) * unit) + 3u;
+    t2[j].y = (unsigned)llrintl((x - t) / (one + t) * unit) + 1u;
   }
 }
 
