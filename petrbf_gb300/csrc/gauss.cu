@@ -18,8 +18,8 @@
 //   3. each warp takes groups of kGroup targets, its lanes stride over the compacted
 //      sources, and the partial sums are reduced with warp shuffles.
 // FP64 form: grids whose windows fit the fixed-point exponents of gauss_fx.cuh take the
-// kernels of gauss_fx.cu; the others (wider than 18 sigma, more than 15 cells across, beyond
-// 65535 cells in y) the kernels here, with exp on the FP64 pipe by a table-folded polynomial
+// kernels of gauss_fx.cu; the others (wider than 18 sigma, in 3D 12, more than 15 cells across,
+// beyond 65535 cells in y) the kernels here, with exp on the FP64 pipe by a table-folded polynomial
 // (12 FP64 instructions per pair, range reduction bits and the 2^-m scaling on the integer
 // pipe); coordinates relative to the cell centre, unscaled, so x_t - x_s rounds as in the
 // reference. FP32 form: scaled FP32 coordinates relative to the cell centre and the SFU exp2.

@@ -134,15 +134,16 @@ inline void fx_tables(uint2* t1, uint2* t2) {
 }
 
 // Whether a grid's sums can take the fixed-point form: the pairs of a target and a source of
-// its truncation set (or of its own cell) differ by less than 16 units per axis and a stays
-// below 512, the scaled coordinates stay below 2^40 units (their products keep 2^-8 of the
-// last place), and sigma is far from the ends of FP64's range.
+// its truncation set (or of its own cell) differ by less than 16 units per axis and 32 units over
+// the axes together (dh dl, below 2^58 a unit of difference, is summed in 63 bits: 18.6 sigma per
+// axis in 2D, 12.4 in 3D) and a stays below 512, the scaled coordinates stay below 2^40 units
+// (their products keep 2^-8 of the last place), and sigma is far from the ends of FP64's range.
 inline bool fx_grid_ok(const Grid& g) {
   if (!(g.sigma > 1e-100 && g.sigma < 1e100)) return false;
   const double unit = std::sqrt(1.0 / (2.0 * g.sigma * g.sigma * 0.6931471805599453));
   const double half = 0.5 * g.box, reach = (g.trunc_len > half ? g.trunc_len : half) + half;
   const double d = reach * unit;
-  if (!(d < 0.99 * 16.0 && g.dim * d * d < 0.98 * 512.0)) return false;
+  if (!(d < 0.99 * 16.0 && g.dim * d < 0.99 * 32.0 && g.dim * d * d < 0.98 * 512.0)) return false;
   const double lo[3] = {g.xmin, g.ymin, g.zmin};
   const int nc[3] = {g.nx, g.ny, g.nz};
   for (int k = 0; k < g.dim; k++) {
