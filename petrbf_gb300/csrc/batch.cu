@@ -165,8 +165,9 @@ std::vector<int2> make_items(const BatchState& B, int tile, long long* pairs) {
   return out;
 }
 
-void upload_items(GaussPlan& P, const std::vector<int2>& items, cudaStream_t s) {
+void upload_items(GaussPlan& P, const std::vector<int2>& items, int tile, cudaStream_t s) {
   P.nitems = (int)items.size();
+  P.max_tile = tile;
   P.items.reserve(std::max<size_t>(items.size(), 1));
   PRBF_CUDA(cudaMemcpyAsync(P.items.get(), items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice, s));
   PRBF_CUDA(cudaStreamSynchronize(s));
@@ -184,7 +185,7 @@ Schedule autotune(Ctx& c, BatchState& B, const double* vin, double* vout, bool f
   for (int tile : tiles) {
     std::vector<int2> all = make_items(B, tile, nullptr), sample;
     for (size_t i = 0; i < all.size(); i += 8) sample.push_back(all[i]);
-    upload_items(B.plan, sample, c.stream);
+    upload_items(B.plan, sample, tile, c.stream);
     for (int grid : grids) {
       B.plan.grid = grid;
       gauss_sum_dev(B.plan, B.op.v, B.op.v, vin, vout, fp32, c.err.get(), c.stream);  // warm-up
@@ -303,7 +304,6 @@ void batch_interpolate(Ctx& c, int nprob, const prbf_problem* probs, int* its_ou
   B.plan.g.cbase = 0;
   B.plan.batched = true;
   B.plan.pairs = pairs;
-  B.plan.max_tile = 128;
   B.plan.grids.reserve(nprob);
   B.plan.cprob.reserve(NC);
   PRBF_CUDA(cudaMemcpyAsync(B.plan.grids.get(), hgrids.data(), sizeof(Grid) * nprob, cudaMemcpyHostToDevice, c.stream));
@@ -392,7 +392,7 @@ void batch_interpolate(Ctx& c, int nprob, const prbf_problem* probs, int* its_ou
     schedule_cache()[key] = sch;
   }
   long long pairs_check = 0;
-  upload_items(B.plan, make_items(B, sch.tile, &pairs_check), c.stream);
+  upload_items(B.plan, make_items(B, sch.tile, &pairs_check), sch.tile, c.stream);
   B.plan.grid = sch.grid;
   // FP64 sums in the symmetric form where it applies (each exponential for both rows of a
   // point pair; the autotuned schedule then serves the FP32 sums of the mixed form)

@@ -114,7 +114,7 @@ struct PointsView {
 struct GaussPlan {
   Grid g;
   int nitems = 0;
-  int max_tile = 0;
+  int max_tile = 0;  // targets of an item at most
   long long pairs = 0;
   int max_trunc = 0;
   int grid = 0;           // CTAs of a launch (0: one per item; fewer: persistent rounds)

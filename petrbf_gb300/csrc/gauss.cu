@@ -131,7 +131,7 @@ struct GaussMinBlocks {
 template <int DIM, bool F32, int NV, bool BATCH>
 __global__ void __launch_bounds__(kThreads, GaussMinBlocks<F32>::v) k_gauss(
     Grid g0, const Grid* __restrict__ grids, const int* __restrict__ cprob, const int2* __restrict__ items, int nitems,
-    const double* __restrict__ tx, const double* __restrict__ ty, const double* __restrict__ tz,
+    int tile, const double* __restrict__ tx, const double* __restrict__ ty, const double* __restrict__ tz,
     const int* __restrict__ cs_t, const double* __restrict__ sx, const double* __restrict__ sy,
     const double* __restrict__ sz, const double* __restrict__ sg, const int* __restrict__ cs_s, double* __restrict__ w,
     long long vstride, SumConsts k0, SegSkip seg, unsigned* err, const int* __restrict__ skip) {
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kThreads, GaussMinBlocks<F32>::v) k_gauss(
     }
     const double scale = kc.scale, kexp = kc.kexp;
     const int cb = g.cbase;
-    const int nt = min(kTileT, cs_t[ic + 1] - t0);
+    const int nt = min(BATCH ? tile : kTileT, cs_t[ic + 1] - t0);
     int ix, iy, iz;
     cell_xyz(g, ic - cb, ix, iy, iz);
     const double xc = centre_coord(g.xmin, ix, g.box);
@@ -530,8 +530,9 @@ struct LayoutF {
 template <int DIM, int NV, bool BATCH>
 __global__ void __launch_bounds__(kThreads, 6) k_gauss_f32m(
     Grid g0, const Grid* __restrict__ grids, const int* __restrict__ cprob, SegSkip seg,
-    const int2* __restrict__ items, int nitems, const double* __restrict__ tx, const double* __restrict__ ty,
-    const double* __restrict__ tz, const int* __restrict__ cs_t, const float* __restrict__ su,
+    const int2* __restrict__ items, int nitems, int tile, const double* __restrict__ tx,
+    const double* __restrict__ ty, const double* __restrict__ tz, const int* __restrict__ cs_t,
+    const float* __restrict__ su,
     const float* __restrict__ sv, const float* __restrict__ sw, const unsigned long long* __restrict__ smask,
     const float* __restrict__ sg, long long vs_g, const int* __restrict__ cs_s, double* __restrict__ w,
     long long vs_w, double scale0, double norm0, unsigned* err, const int* __restrict__ skip, VecSkip left) {
@@ -579,7 +580,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_gauss_f32m(
     const int cb = g.cbase;
     const float boxs = (float)(g.box * scale);
     const int nb = g.nb_trunc;
-    const int nt = min(kTileT, cs_t[ic + 1] - t0);
+    const int nt = min(BATCH ? tile : kTileT, cs_t[ic + 1] - t0);
     int ix, iy, iz;
     cell_xyz(g, ic - cb, ix, iy, iz);
     const double xc = centre_coord(g.xmin, ix, g.box);
@@ -1489,7 +1490,7 @@ void launch(const GaussPlan& P, const PointsView& t, const PointsView& s, const 
   const SumConsts k0 = sum_consts(P.g.sigma, F32, ExpTab<UseBigTab<DIM, NV>::v>::n);
   const int grid = P.grid > 0 ? std::min(P.grid, P.nitems) : P.nitems;
   k_gauss<DIM, F32, NV, BATCH><<<grid, kThreads, sm, st>>>(P.g, P.grids.get(), P.cprob.get(), P.items.get(), P.nitems,
-                                                           t.x, t.y, t.z, t.cell_start, s.x, s.y, s.z, gv,
+                                                           P.max_tile, t.x, t.y, t.z, t.cell_start, s.x, s.y, s.z, gv,
                                                            s.cell_start, w, vstride, k0, P.seg, err, skip);
   PRBF_CHECK_LAUNCH();
 }
@@ -1574,8 +1575,8 @@ void launch_f32m(const GaussPlan& P, const PointsView& t, const PointsView& s, c
   const SumConsts k0 = sum_consts(P.g.sigma, true, 0);
   const int grid = P.grid > 0 ? std::min(P.grid, P.nitems) : P.nitems;
   k_gauss_f32m<DIM, NV, BATCH><<<grid, kThreads, sm, st>>>(
-      P.g, P.grids.get(), P.cprob.get(), P.seg, P.items.get(), P.nitems, t.x, t.y, t.z, t.cell_start, P.su.get(),
-      P.sv.get(), P.sw.get(), P.smask.get(), P.g32.get(), P.g32_stride, s.cell_start, w, vstride, k0.scale, k0.norm,
+      P.g, P.grids.get(), P.cprob.get(), P.seg, P.items.get(), P.nitems, P.max_tile, t.x, t.y, t.z, t.cell_start,
+      P.su.get(), P.sv.get(), P.sw.get(), P.smask.get(), P.g32.get(), P.g32_stride, s.cell_start, w, vstride, k0.scale, k0.norm,
       err, skip, left);
   PRBF_CHECK_LAUNCH();
 }

@@ -147,7 +147,7 @@ struct FxArgs {
   double* w;
   double* part;
   long long pstride;
-  int K, n, ncs;
+  int K, n, ncs, tile;
   VecSkip left;
 };
 
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(kFxThreads<SYM>, 2) k_gauss_fx(Grid g0, const 
       if (seg.cell_done(ic)) continue;  // a stopped problem (uniform over the CTA)
       g = grids[cprob[ic]];
     }
-    const int nt_all = min(kTileT, cs_t[ic + 1] - t0);
+    const int nt_all = min(BATCH ? a.tile : kTileT, cs_t[ic + 1] - t0);
     const int passes = (nt_all + TT - 1) / TT;
     const double norm = g.norm;
     for (int q = blockIdx.y; q < passes; q += gridDim.y) {
@@ -677,7 +677,7 @@ void launch_fx(const GaussPlan& P, const PointsView& t, const PointsView& s, con
   }
   const DevBuf<uint2>* T = P.fx_self ? P.fxs : P.fxt;
   FxArgs a{T[0].get(), T[1].get(), T[2].get(), P.fxs[0].get(), P.fxs[1].get(), P.fxs[2].get(), P.smask.get(), gv,
-           vstride,    w,          nullptr,    0,              0,              s.n,            P.fx_ncs, left};
+           vstride,    w,          nullptr,    0,              0,              s.n,            P.fx_ncs, P.max_tile, left};
   const int2* items = P.items.get();
   int nitems = P.nitems, grid = P.grid;
   if constexpr (SYM) {
@@ -687,6 +687,7 @@ void launch_fx(const GaussPlan& P, const PointsView& t, const PointsView& s, con
     if (P.sym_nitems > 0) {  // a batch's list of one item per cell
       items = P.sym_items.get();
       nitems = P.sym_nitems;
+      a.tile = kTileT;
       grid = 0;
     }
   }
