@@ -2102,6 +2102,10 @@ void rasm_factor(RasmPlan& R, const BlockGeom& G, const std::vector<int>& hcnt, 
     long long nslot = 0;
     for (int c = 0; c < ncell; c++) nslot += hcnt[c];
     R.nslot = nslot;
+    // slots of several FP64 vectors only where they fit the workspace's budget (one vector's are
+    // what the method needs)
+    if (!fp32)
+      while (R.max_nv > 1 && (double)nslot * R.max_nv * sizeof(double) > ws_budget_bytes) R.max_nv--;
     R.Y.reserve(std::max<long long>(nslot, 1) * std::max(1, std::min(4, R.max_nv)));
     R.inv_off.reserve((size_t)G.n + 1);
     R.inv_slot.reserve(std::max<long long>(nslot, 1));
