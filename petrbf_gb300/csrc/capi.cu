@@ -199,6 +199,9 @@ int prbf_ctx_create(const prbf_params* p, prbf_ctx** out) {
     int st = e.status;
     delete ctx;  // (outside of any scope: its buffers are freed)
     return st;
+  } catch (const std::bad_alloc&) {
+    delete ctx;
+    return PRBF_ERR_CAPACITY;
   }
   *out = ctx;
   return PRBF_OK;
@@ -217,7 +220,11 @@ int prbf_ctx_destroy(prbf_ctx* ctx) {
 long long prbf_memory_kept(int device) { return (long long)dev_pool_kept(device); }
 
 int prbf_memory_release(int device) {
-  dev_pool_trim(device);
+  try {
+    dev_pool_trim(device);
+  } catch (const std::bad_alloc&) {
+    return PRBF_ERR_CAPACITY;
+  }
   return PRBF_OK;
 }
 

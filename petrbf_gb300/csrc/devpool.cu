@@ -70,6 +70,7 @@ int current_device() {
 // Takes the device's cached blocks out (all, or those unused for long), for the caller to free.
 std::vector<void*> take(DevicePool& D, bool all) {
   std::vector<void*> out;
+  out.reserve(D.free.size());  // (whatever fails, fails before a block is taken out)
   for (auto it = D.free.begin(); it != D.free.end();)
     if (all || D.epoch - it->second.since > kKeep) {
       out.push_back(it->second.p);
@@ -130,9 +131,9 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
     }
     if (best != r.second) {
       *p = best->second.p;
+      P.used[*p] = {d, cls};
       D.cached -= cls;
       D.free.erase(best);
-      P.used[*p] = {d, cls};
       return cudaSuccess;
     }
   }
@@ -143,8 +144,13 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
     return cudaMalloc(p, bytes);  // (as asked for; not the pool's)
   }
   if (e == cudaSuccess) {
-    std::lock_guard<std::mutex> lk(P.m);
-    P.used[*p] = {d, cls};
+    try {
+      std::lock_guard<std::mutex> lk(P.m);
+      P.used[*p] = {d, cls};
+    } catch (const std::bad_alloc&) {
+      cudaFree(*p);
+      throw;
+    }
   }
   return e;
 }
@@ -177,11 +183,16 @@ void dev_pool_stream_done(int device, cudaStream_t s) {
   std::vector<void*> old;
   {
     std::lock_guard<std::mutex> lk(P.m);
-    DevicePool& D = P.dev[device];
+    const auto it = P.dev.find(device);
+    if (it == P.dev.end()) return;
+    DevicePool& D = it->second;
     D.epoch++;
     for (auto& f : D.free)
       if (f.second.stream == s) f.second.stream = nullptr;
-    old = take(D, false);
+    try {
+      old = take(D, false);
+    } catch (const std::bad_alloc&) {  // (they go another time)
+    }
   }
   for (void* p : old) cudaFree(p);
 }
@@ -191,7 +202,8 @@ void dev_pool_trim(int device) {
   std::vector<void*> all;
   {
     std::lock_guard<std::mutex> lk(P.m);
-    all = take(P.dev[device], true);
+    const auto it = P.dev.find(device);
+    if (it != P.dev.end()) all = take(it->second, true);
   }
   for (void* p : all) cudaFree(p);
 }
@@ -199,7 +211,8 @@ void dev_pool_trim(int device) {
 size_t dev_pool_kept(int device) {
   Pool& P = pool();
   std::lock_guard<std::mutex> lk(P.m);
-  return P.dev[device].cached;
+  const auto it = P.dev.find(device);
+  return it == P.dev.end() ? 0 : it->second.cached;
 }
 
 size_t dev_mem_free() {

@@ -16,6 +16,14 @@ SOURCE = r"""
 #include <vector>
 #include "devpool.cu"
 using namespace prbf;
+static bool fail_new = false;
+void* operator new(size_t n) {
+  void* p = fail_new ? nullptr : std::malloc(n ? n : 1);
+  if (!p) throw std::bad_alloc();
+  return p;
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 static const size_t MB = (size_t)1 << 20, GB = (size_t)1 << 30;
 static std::map<void*, size_t> live;   // what the driver has given out
 static size_t taken = 0, capacity = 64 * GB;
@@ -111,6 +119,28 @@ int main() {
     { StreamScope sc(s1); a = get(MB); }
     { StreamScope sc(s1, true); dev_free(a); }
     { StreamScope sc(s2); CHECK(get(MB) == a); dev_free(a); }
+  }
+  {  // no host memory: nothing is thrown at a destructor, nothing is lost
+    StreamScope sc(s1);
+    void *a = get(5 * MB), *b = get(6 * MB);
+    dev_free(b);
+    const size_t t = taken;
+    fail_new = true;
+    dev_free(a);  // (to the driver: it cannot be kept)
+    dev_pool_stream_done(0, s2);
+    fail_new = false;
+    CHECK(taken == t - 5 * MB);
+    fail_new = true;
+    bool thrown = false;
+    try {
+      a = get(7 * MB);
+    } catch (const std::bad_alloc&) {
+      thrown = true;
+    }
+    fail_new = false;
+    CHECK(thrown && taken == t - 5 * MB);
+    CHECK(get(6 * MB) == b);
+    dev_free(b);
   }
   CHECK(dev_pool_kept(7) == 0);
   dev_pool_trim(0);
