@@ -38,8 +38,18 @@
 namespace prbf {
 namespace {
 
+constexpr int kThreads = 128;  // 4 warps
+constexpr int kWarps = kThreads / 32;
 constexpr int kGroup = 4;      // targets per warp pass
+constexpr int kMaxPieces = 64; // source ranges per fill
+constexpr int kMaxRanges = 256; // column ranges of an item kept in shared memory
 constexpr int kRawCap = 1024;  // staged raw sources per fill (incl. alignment padding)
+
+struct Piece {
+  int raw_off;  // smem index of the first valid element
+  int count;    // valid elements
+  int gstart;   // global (sorted) index of the first valid element
+};
 
 // exp table: e^a with a = -L*d, d >= 0, L = ln2/n:  k = rint(d), r = k - d in [-1/2, 1/2],
 // e^a = 2^(-k/n) e^(L r) = 2^-m T[j] p(r),  k = m*n + j; the table holds T[j] c_i

@@ -4,17 +4,7 @@
 
 namespace prbf {
 
-constexpr int kThreads = 128;   // 4 warps
-constexpr int kWarps = kThreads / 32;
-constexpr int kTileT = 128;     // targets per work item
-constexpr int kMaxPieces = 64;  // source ranges per fill
-constexpr int kMaxRanges = 256; // column ranges of an item kept in shared memory
-
-struct Piece {
-  int raw_off;  // smem index of the first valid element
-  int count;    // valid elements
-  int gstart;   // global (sorted) index of the first valid element
-};
+constexpr int kTileT = 128;  // targets per work item
 
 constexpr size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
 

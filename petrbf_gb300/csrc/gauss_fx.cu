@@ -12,10 +12,11 @@
 // (bulk copies on an mbarrier, the next piece in flight while one is filtered), keeps those of
 // the cell's truncation set in order, and hands them on in two buffers of CfgX::KC sources. The
 // consumer warps own an even share of the pass's targets, at most CfgX::TG each, whose sums
-// stay in registers; their lanes stride over a buffer's sources. Nothing but the buffers' mbarriers joins the warps: with CTA barriers around the
-// filtering they spent a fifth of their time waiting there.
+// stay in registers; their lanes stride over a buffer's sources. Nothing but the buffers'
+// mbarriers joins the warps: with CTA barriers around the filtering they spent a fifth of their
+// time waiting there.
 // Measured against the FP64-pipe kernels of gauss.cu (one product, caller order): 2D, 4x10^6
-// points 44.7 -> 7.9 ms (79.8 -> 450 Gpairs/s); 3D, 96^3 points 180.7 -> 18.7 ms (39.5 -> 381).
+// points 44.7 -> 7.9 ms (79.8 -> 450 Gpairs/s); 3D, 96^3 points 180.7 -> 17.8 ms (39.5 -> 400).
 // What bounds it: the FP64 accumulations take 16 of the 23 (2D) to 27 (3D) clocks an SM spends
 // per 32 pairs; the shared-memory lookups (14), the integer pipes (10 to 13) and the issue of
 // about 50 instructions (12) overlap with them, 24 warps an SM not hiding all of it.
@@ -27,7 +28,7 @@
 // row j's share into per-warp sums in shared memory; another warp puts their totals into
 // part[pass][o][j], o the window offset (one writer per slot), for k_sym_gather to add to the
 // rows. A pair of rows then costs one exponential and two fused multiply-adds, and the FP64
-// pipe bounds it (89 % busy; a fifth of that is the row-j totals, the trees that end the
+// pipe bounds it (85 % busy; a fifth of that is the row-j totals, the trees that end the
 // targets' sums and lanes past a buffer's end).
 #include <algorithm>
 #include <atomic>

@@ -124,26 +124,22 @@ __global__ void k_split_hl(long long n, const double* __restrict__ v, float2* __
   }
 }
 
-// K[i][j] = exp(-|x_a - x_b|^2 / (2 sigma^2)) (+ shift on the diagonal), block order
-// neighbours first then centre: block row i < n1 -> buffer entry nc + i, else i - n1.
-// Lower triangle only (the factorisation reads nothing else). hl (FP32 form): the n
-// points' coordinates split by k_split_hl, dim arrays of n one after the other. FP64 form:
-// the differences as the reference forms them (x_a - x_b), |d|^2 = fma(dy, dy, dx dx)
-// (+ fma(dz, dz, .)), and the exponential of the sums' table (exp_neg_tab, kexp = 1024 /
-// (2 sigma^2 ln2)), every operation rounded as written.
-// FP32 rows of the block assembly: one warp, lanes along row i (columns 0..i), the split
-// coordinates from shared memory, the exponential as the FP32 sums take it (ex2.approx);
-// the diagonal shift is added by the lane that wrote the diagonal.
 // FP32 blocks as the tensor-core factorisation reads them (k_chol_tc).
 // Row pitch (floats) of a block of nbp rows in memory: whole 128-byte lines.
 __host__ __device__ __forceinline__ int tc_pitch(int nbp) { return (nbp + 31) & ~31; }
 // S_c form: empty rows and columns between the neighbours (n1) and the centre points.
 __host__ __device__ __forceinline__ int tc_pad(int n1) { return -n1 & 3; }
+
 __device__ __forceinline__ float asm_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+
+// FP32 rows of the block assembly: one warp, lanes along row i (columns 0..i), the split
+// coordinates from shared memory, the exponential as the FP32 sums take it (ex2.approx);
+// the diagonal shift is added by the lane that wrote the diagonal. Columns from nl on move by
+// pad.
 template <int DIM>
 __device__ __forceinline__ void asm_row_f32(float* __restrict__ Arow, const float2* s_hl, int nbk, int i, float c2,
                                             float sh, int lane, int nl, int pad) {
@@ -163,6 +159,13 @@ __device__ __forceinline__ void asm_row_f32(float* __restrict__ Arow, const floa
   if (sh != 0.f && lane == (i & 31)) Arow[i < nl ? i : i + pad] += sh;
 }
 
+// K[i][j] = exp(-|x_a - x_b|^2 / (2 sigma^2)) (+ shift on the diagonal), block order
+// neighbours first then centre: block row i < n1 -> buffer entry nc + i, else i - n1.
+// Lower triangle only (the factorisation reads nothing else). hl (FP32 form): the n
+// points' coordinates split by k_split_hl, dim arrays of n one after the other. FP64 form:
+// the differences as the reference forms them (x_a - x_b), |d|^2 = fma(dy, dy, dx dx)
+// (+ fma(dz, dz, .)), and the exponential of the sums' table (exp_neg_tab, kexp = 1024 /
+// (2 sigma^2 ln2)), every operation rounded as written.
 template <class T>
 __global__ void k_assemble(int nblk, const int* __restrict__ blk_cell, const long long* __restrict__ boff,
                            const int* __restrict__ cs, const int* __restrict__ idx,

@@ -79,9 +79,9 @@ void rasm_factor_rows(const RasmPlan& R, int cell, int nb, double* out, cudaStre
 // Sets the dynamic shared memory limit of the apply kernel for this plan.
 void rasm_set_apply_smem(const RasmPlan& R);
 // Restricted: out[centre(c)] = (A_c^-1 r[buffer(c)])[centre] for every cell; basic:
-// out = sum_c R_c^T A_c^-1 R_c r (sorted order, n entries).
-// left: the vectors of stopped systems left out. nv vectors at stride vstride (applied up to min(4, R.max_nv) at a time; the factor is
-// read once per launch for all of them).
+// out = sum_c R_c^T A_c^-1 R_c r (sorted order, n entries). nv vectors at stride vstride
+// (applied up to min(4, R.max_nv) at a time; the factor is read once per launch for all of
+// them); left: those of stopped systems left out.
 void rasm_apply(const RasmPlan& R, const int* cs, const double* r, double* out, cudaStream_t s,
                 const int* skip = nullptr, int nv = 1, long long vstride = 0, VecSkip left = VecSkip{});
 
