@@ -135,6 +135,7 @@ struct GaussPlan {
   // targets' where they are another point set
   bool fx_ready = false;
   bool fx_self = true;
+  bool fx_wide = false;  // fx_grid_wide
   int fx_ncs = 0;       // entries of the cell starts
   DevBuf<uint2> fxs[3], fxt[3];
   // FP64 matvec with each exponential used for both rows (targets == sources, every cell

@@ -18,7 +18,7 @@
 //   3. each warp takes groups of kGroup targets, its lanes stride over the compacted
 //      sources, and the partial sums are reduced with warp shuffles.
 // FP64 form: grids whose windows fit the fixed-point exponents of gauss_fx.cuh take the
-// kernels of gauss_fx.cu; the others (wider than 18 sigma, in 3D 12, more than 15 cells across,
+// kernels of gauss_fx.cu; the others (wider than 18 sigma, in 3D 15, more than 15 cells across,
 // beyond 65535 cells in y) the kernels here, with exp on the FP64 pipe by a table-folded polynomial
 // (12 FP64 instructions per pair, range reduction bits and the 2^-m scaling on the integer
 // pipe); coordinates relative to the cell centre, unscaled, so x_t - x_s rounds as in the
@@ -1726,6 +1726,7 @@ void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& sr
     if (fx) {
       gauss_fx_upload_tables(s);
       plan.fx_self = self;
+      plan.fx_wide = fx_grid_wide(g);
       plan.fx_ncs = g.ncell + 1;
       if (!self) {
         PointForms ot;
@@ -1835,10 +1836,12 @@ void gauss_plan_forms_batch(GaussPlan& plan, const std::vector<Grid>& grids, con
   plan.f32_ready = plan.fx_ready = false;
   if (src.n <= 0) return;
   bool fx = forms & FORM_F64;
+  plan.fx_wide = false;
   int ncell = 0;
   for (const Grid& g : grids) {
     if (!f32_grid_ok(g)) return;
     fx = fx && fx_grid_ok(g);
+    plan.fx_wide = plan.fx_wide || fx_grid_wide(g);
     ncell += g.ncell;
   }
   const bool f32 = forms & FORM_F32;

@@ -87,10 +87,10 @@ struct LayoutX {
 };
 
 // exp of a pair: coordinates (l, h) of target and source
-template <int DIM>
+template <int DIM, bool WIDE>
 __device__ __forceinline__ double fx_pair(const uint2 (&t)[DIM], const uint2 (&s)[DIM], const uint2* t1,
                                           const uint2* t2) {
-  const unsigned long long B = fx_exponent<DIM>(t, s);
+  const unsigned long long B = fx_exponent<DIM, WIDE>(t, s);
   const unsigned bh = (unsigned)(B >> 32);
   const uint2 p = t1[(bh >> 11) & 2047u], q = t2[bh & 2047u];
   return __longlong_as_double((long long)fx_pow2_bits(bh, (unsigned)B, p, q));
@@ -154,7 +154,7 @@ struct FxArgs {
 
 // One pass of a consumer warp with N targets from t: buffers until the last one. Returns false
 // when a wait gave up.
-template <int DIM, int NV, bool SYM, int N>
+template <int DIM, int NV, bool SYM, bool WIDE, int N>
 __device__ __forceinline__ bool fx_consume(unsigned char* smem, FxShared& sh, const FxArgs& a, const int (&vm)[NV],
                                            int t, double norm, int wid, int lane, int& b, unsigned& ph) {
   using Lay = LayoutX<DIM, NV, SYM>;
@@ -249,7 +249,7 @@ __device__ __forceinline__ bool fx_consume(unsigned char* smem, FxShared& sh, co
           }
 #pragma unroll
           for (int k = 0; k < CNT; k++) {
-            const double e = fx_pair<DIM>(tc[k], sc, t1, t2);
+            const double e = fx_pair<DIM, WIDE>(tc[k], sc, t1, t2);
 #pragma unroll
             for (int v = 0; v < NV; v++) acc[v][K0 + k] = fma(g[v], e, acc[v][K0 + k]);
             // row j, when target k is in T(c(j)): both its bits at c(j)'s offset
@@ -318,7 +318,7 @@ __device__ __forceinline__ void fx_sym_range(const Grid& g, const int* __restric
   pb = cs[ca + (jy1 - y0) + 1];
 }
 
-template <int DIM, int NV, bool BATCH, bool SYM>
+template <int DIM, int NV, bool BATCH, bool SYM, bool WIDE>
 __global__ void __launch_bounds__(kFxThreads<SYM>, 2) k_gauss_fx(Grid g0, const Grid* __restrict__ grids,
                                                            const int* __restrict__ cprob, SegSkip seg,
                                                            const int2* __restrict__ items, int nitems,
@@ -405,18 +405,18 @@ __global__ void __launch_bounds__(kFxThreads<SYM>, 2) k_gauss_fx(Grid g0, const 
         const int t = t0 + ta + u0;
         bool ok;
         switch (cnt) {
-          case 0: ok = fx_consume<DIM, NV, SYM, 0>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
-          case 1: ok = fx_consume<DIM, NV, SYM, 1>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
-          case 2: ok = fx_consume<DIM, NV, SYM, 2>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
-          case 3: ok = fx_consume<DIM, NV, SYM, 3>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
-          case 4: ok = fx_consume<DIM, NV, SYM, 4>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+          case 0: ok = fx_consume<DIM, NV, SYM, WIDE, 0>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+          case 1: ok = fx_consume<DIM, NV, SYM, WIDE, 1>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+          case 2: ok = fx_consume<DIM, NV, SYM, WIDE, 2>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+          case 3: ok = fx_consume<DIM, NV, SYM, WIDE, 3>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+          case 4: ok = fx_consume<DIM, NV, SYM, WIDE, 4>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
           default:
             if constexpr (C::TG == 8) {
               switch (cnt) {
-                case 5: ok = fx_consume<DIM, NV, SYM, 5>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
-                case 6: ok = fx_consume<DIM, NV, SYM, 6>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
-                case 7: ok = fx_consume<DIM, NV, SYM, 7>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
-                default: ok = fx_consume<DIM, NV, SYM, 8>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+                case 5: ok = fx_consume<DIM, NV, SYM, WIDE, 5>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+                case 6: ok = fx_consume<DIM, NV, SYM, WIDE, 6>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+                case 7: ok = fx_consume<DIM, NV, SYM, WIDE, 7>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
+                default: ok = fx_consume<DIM, NV, SYM, WIDE, 8>(smem, sh, a, vm, t, norm, wid, lane, b, ph); break;
               }
             } else {
               ok = false;  // (not reached: at most TG targets a warp)
@@ -663,8 +663,8 @@ __global__ void __launch_bounds__(kFxThreads<SYM>, 2) k_gauss_fx(Grid g0, const 
   }
 }
 
-template <int DIM, int NV, bool BATCH, bool SYM>
-void launch_fx(const GaussPlan& P, const PointsView& t, const PointsView& s, const double* gv, double* w,
+template <int DIM, int NV, bool BATCH, bool SYM, bool WIDE>
+void launch_fx_k(const GaussPlan& P, const PointsView& t, const PointsView& s, const double* gv, double* w,
                long long vstride, unsigned* err, const int* skip, VecSkip left, cudaStream_t st) {
   constexpr size_t sm = LayoutX<DIM, NV, SYM>::total;
   static_assert(sm <= 112 * 1024, "two CTAs of k_gauss_fx per SM");
@@ -672,7 +672,7 @@ void launch_fx(const GaussPlan& P, const PointsView& t, const PointsView& s, con
   int dev = 0;
   PRBF_CUDA(cudaGetDevice(&dev));
   if (dev >= 64 || !attr_set[dev]) {
-    PRBF_CUDA(cudaFuncSetAttribute(k_gauss_fx<DIM, NV, BATCH, SYM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    PRBF_CUDA(cudaFuncSetAttribute(k_gauss_fx<DIM, NV, BATCH, SYM, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)sm));
     if (dev < 64) attr_set[dev] = true;
   }
@@ -697,9 +697,17 @@ void launch_fx(const GaussPlan& P, const PointsView& t, const PointsView& s, con
   grid = grid > 0 ? std::min(grid, nitems) : nitems;
   // few items: a cell's passes on CTAs of their own
   const dim3 gd(grid, nitems < kResident ? ceil_div(kTileT, CfgX<DIM, NV, SYM>::TT) : 1);
-  k_gauss_fx<DIM, NV, BATCH, SYM><<<gd, kFxThreads<SYM>, sm, st>>>(P.g, P.grids.get(), P.cprob.get(), P.seg, items,
+  k_gauss_fx<DIM, NV, BATCH, SYM, WIDE><<<gd, kFxThreads<SYM>, sm, st>>>(P.g, P.grids.get(), P.cprob.get(), P.seg, items,
                                                                nitems, t.cell_start, s.cell_start, a, err, skip);
   PRBF_CHECK_LAUNCH();
+}
+
+template <int DIM, int NV, bool BATCH, bool SYM>
+void launch_fx(const GaussPlan& P, const PointsView& t, const PointsView& s, const double* gv, double* w,
+               long long vstride, unsigned* err, const int* skip, VecSkip left, cudaStream_t st) {
+  if constexpr (DIM == 3)
+    if (P.fx_wide) return launch_fx_k<DIM, NV, BATCH, SYM, true>(P, t, s, gv, w, vstride, err, skip, left, st);
+  launch_fx_k<DIM, NV, BATCH, SYM, false>(P, t, s, gv, w, vstride, err, skip, left, st);
 }
 
 template <int DIM>

@@ -59,8 +59,9 @@ __host__ __device__ __forceinline__ unsigned long long fx_pow2_bits(unsigned bh,
   return (V >> 10) + X + ((unsigned long long)((bh >> 2) & 0x3ff00000u) << 32);
 }
 
-// B of a pair: coordinates (l, h) of target and source.
-template <int DIM>
+// B of a pair: coordinates (l, h) of target and source. WIDE (fx_grid_wide): the last axis' low
+// product by itself, where the sum of all three could pass 63 bits.
+template <int DIM, bool WIDE = false>
 __host__ __device__ __forceinline__ unsigned long long fx_exponent(const uint2 (&t)[DIM], const uint2 (&s)[DIM]) {
   long long A = -kFxBias, C = 0;  // C carries the minus sign of B
 #ifdef __CUDA_ARCH__
@@ -69,7 +70,10 @@ __host__ __device__ __forceinline__ unsigned long long fx_exponent(const uint2 (
   for (int d = 0; d < DIM; d++) {
     const int dh = (int)(t[d].y - s[d].y), dl = (int)(s[d].x - t[d].x);
     A += (long long)dh * dh;
-    C += (long long)dh * dl;
+    if (WIDE && d == DIM - 1)
+      A -= (long long)dh * dl >> 30;
+    else
+      C += (long long)dh * dl;
   }
   return (unsigned long long)((C >> 30) - A);
 }
@@ -133,17 +137,25 @@ inline void fx_tables(uint2* t1, uint2* t2) {
   }
 }
 
-// Whether a grid's sums can take the fixed-point form: the pairs of a target and a source of
-// its truncation set (or of its own cell) differ by less than 16 units per axis and 32 units over
-// the axes together (dh dl, below 2^58 a unit of difference, is summed in 63 bits: 18.6 sigma per
-// axis in 2D, 12.4 in 3D) and a stays below 512, the scaled coordinates stay below 2^40 units
-// (their products keep 2^-8 of the last place), and sigma is far from the ends of FP64's range.
-inline bool fx_grid_ok(const Grid& g) {
-  if (!(g.sigma > 1e-100 && g.sigma < 1e100)) return false;
+// The largest difference per axis, in units of the scaled coordinate, of a target and a source of
+// its truncation set (or of its own cell).
+inline double fx_reach(const Grid& g) {
   const double unit = std::sqrt(1.0 / (2.0 * g.sigma * g.sigma * 0.6931471805599453));
   const double half = 0.5 * g.box, reach = (g.trunc_len > half ? g.trunc_len : half) + half;
-  const double d = reach * unit;
-  if (!(d < 0.99 * 16.0 && g.dim * d < 0.99 * 32.0 && g.dim * d * d < 0.98 * 512.0)) return false;
+  return reach * unit;
+}
+
+// Whether the low products' sum could pass 63 bits: dh dl is below 2^58 a unit of difference, and
+// the axes together reach 32 units (3D windows beyond 12.4 sigma per axis).
+inline bool fx_grid_wide(const Grid& g) { return !(g.dim * fx_reach(g) < 0.99 * 32.0); }
+
+// Whether a grid's sums can take the fixed-point form: the pairs differ by less than 16 units per
+// axis and a stays below 512, the scaled coordinates stay below 2^40 units (their products keep
+// 2^-8 of the last place), and sigma is far from the ends of FP64's range.
+inline bool fx_grid_ok(const Grid& g) {
+  if (!(g.sigma > 1e-100 && g.sigma < 1e100)) return false;
+  const double unit = std::sqrt(1.0 / (2.0 * g.sigma * g.sigma * 0.6931471805599453)), d = fx_reach(g);
+  if (!(d < 0.99 * 16.0 && g.dim * d * d < 0.98 * 512.0)) return false;
   const double lo[3] = {g.xmin, g.ymin, g.zmin};
   const int nc[3] = {g.nx, g.ny, g.nz};
   for (int k = 0; k < g.dim; k++) {

@@ -28,12 +28,14 @@ static Grid grid(int dim, double sigma, double box, double trunc) {  // widths i
   g.trunc_len = trunc * sigma / 2;
   return g;
 }
-template <int DIM>
+// WIDE: the widest truncation box that the rule takes; else the widest that is not wide
+template <int DIM, bool WIDE>
 static void corners(double sigma, double box) {
-  double lo = 0, hi = 60;  // the widest truncation box that the rule takes
+  double lo = 0, hi = 60;
   for (int i = 0; i < 60; i++) {
     const double mid = 0.5 * (lo + hi);
-    (fx_grid_ok(grid(DIM, sigma, box, mid)) ? lo : hi) = mid;
+    const Grid g = grid(DIM, sigma, box, mid);
+    (fx_grid_ok(g) && (WIDE || !fx_grid_wide(g)) ? lo : hi) = mid;
   }
   const double reach = 0.5 * (std::fmax(lo, box) + box) * sigma;
   const FxScale fs = fx_scale(sigma);
@@ -51,7 +53,7 @@ static void corners(double sigma, double box) {
       d2 += ((long double)a - b) * ((long double)a - b);
     }
     const long double ref = expl(-d2 / (2.0L * sigma * sigma));
-    const unsigned long long B = fx_exponent<DIM>(t, s);
+    const unsigned long long B = WIDE ? fx_exponent<DIM, true>(t, s) : fx_exponent<DIM>(t, s);
     const unsigned bh = (unsigned)(B >> 32);
     const unsigned long long u = fx_pow2_bits(bh, (unsigned)B, t1[(bh >> 11) & 2047], t2[bh & 2047]);
     double v;
@@ -64,8 +66,9 @@ static void corners(double sigma, double box) {
 int main() {
   fx_tables(t1, t2);
   for (double box : {1.0, 3.0, 8.0}) {
-    corners<2>(0.0125, box);
-    corners<3>(0.026, box);
+    corners<2, false>(0.0125, box);
+    corners<3, false>(0.026, box);
+    corners<3, true>(0.026, box);
   }
   return 0;
 }
@@ -83,9 +86,9 @@ def test_corners_of_the_widest_windows(tmp_path):
                     os.path.join(ROOT, "petrbf_gb300", "csrc"), src, "-o", exe], check=True)
     out = subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split("\n")
     rows = [[float(v) for v in ln.split()] for ln in out if ln]
-    assert len(rows) == 6
+    assert len(rows) == 9
     for k, (reach, worst) in enumerate(rows):
-        assert reach > (18 if k % 2 == 0 else 12)  # sigma per axis
+        assert reach > (18, 12, 15)[k % 3]  # sigma per axis: 2D, 3D, 3D wide
         # as for nearer pairs: the power's error, one unit of 2^-54 for the shift and for each
         # axis' squared low parts, the coordinates' half units of 2^-58 times twice the distance
         assert worst <= 3 * 2.0 ** -52 + 9 * 0.6931 * 2.0 ** -54

@@ -8,8 +8,9 @@ from test_gpu_fx_sums import _check
 pytestmark = pytest.mark.gpu
 
 
-# 12.4 sigma per axis, half a cell included: between sigma_trunc 21 and 22 with cells of 3 sigma
-@pytest.mark.parametrize("nt", [20, 21, 22, 23, 25])
+# from 12.4 sigma per axis (half a cell included; between sigma_trunc 21 and 22 with cells of 3
+# sigma) the wide form, from 15.2 (27 and 28) the FP64 pipe's kernels
+@pytest.mark.parametrize("nt", [20, 21, 22, 23, 25, 27, 28])
 def test_3d_windows_at_the_rules_limit(nt):
     rng = np.random.default_rng(nt)
     k = rng.uniform(0.0, 0.9, (1500, 3))
