@@ -448,17 +448,18 @@ struct PointForms {  // null: not wanted
   uint2 *fx = nullptr, *fy = nullptr, *fz = nullptr;
 };
 
-// A warp per cell (of one grid, or of a batch's: cell -> problem -> grid): its lanes stride
-// over the cell's points, the centres of the cells at offsets -nb .. nb computed once.
-// Bound by the FP64 pipe (the box tests): 4x10^6 points in 2D.
+// NL lanes per cell (of one grid, or of a batch's: cell -> problem -> grid): they stride over the
+// cell's points, the centres of the cells at offsets -nb .. nb computed once. Bound by the FP64
+// pipe (the box tests): 4x10^6 points in 2D.
+template <int NL>
 __global__ void __launch_bounds__(256) k_point_forms(Grid g0, const Grid* __restrict__ grids,
                                                      const int* __restrict__ cprob, int ncell,
                                                      const int* __restrict__ cs, const double* __restrict__ x,
                                                      const double* __restrict__ y, const double* __restrict__ z,
                                                      PointForms o) {
-  __shared__ double s_ctr[8][3][kMaskBits];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * 8 + wid;
+  __shared__ double s_ctr[256 / NL][3][kMaskBits];
+  const int wid = threadIdx.x / NL, lane = threadIdx.x % NL;
+  const int c = blockIdx.x * (256 / NL) + wid;
   if (c >= ncell) return;
   const int a = cs[c], b = cs[c + 1];
   if (a == b) return;
@@ -468,18 +469,18 @@ __global__ void __launch_bounds__(256) k_point_forms(Grid g0, const Grid* __rest
   int ix, iy, iz;
   cell_xyz(g, c - g.cbase, ix, iy, iz);
   if (o.mask) {
-    for (int q = lane; q < W; q += 32) {  // bit q: the target cell at offset q - nb from this one
+    for (int q = lane; q < W; q += NL) {  // bit q: the target cell at offset q - nb from this one
       s_ctr[wid][0][q] = centre_coord(g.xmin, ix - (q - nb), g.box);
       s_ctr[wid][1][q] = centre_coord(g.ymin, iy - (q - nb), g.box);
       s_ctr[wid][2][q] = g.dim == 3 ? centre_coord(g.zmin, iz - (q - nb), g.box) : 0.0;
     }
-    __syncwarp();
+    __syncwarp((0xffffffffu >> (32 - NL)) << (threadIdx.x & 31 & ~(NL - 1)));
   }
   const double xc = centre_coord(g.xmin, ix, g.box), yc = centre_coord(g.ymin, iy, g.box);
   const double zc = g.dim == 3 ? centre_coord(g.zmin, iz, g.box) : 0.0;
   const double scale = o.u ? sum_consts(g.sigma, true, 0).scale : 0.0;
   const FxScale fs = o.fx ? fx_scale(g.sigma) : FxScale{0.0, 0.0};
-  for (int j = a + lane; j < b; j += 32) {
+  for (int j = a + lane; j < b; j += NL) {
     const double px = x[j], py = y[j], pz = g.dim == 3 ? z[j] : 0.0;
     if (o.mask) {
       unsigned long long m = (unsigned long long)iy << kMaskCellY;
@@ -1672,6 +1673,18 @@ static PointForms alloc_forms(GaussPlan& plan, int dim, int n, bool f32, bool fx
   return o;
 }
 
+// A warp per cell, or four lanes where the cells hold fewer than 16 points on average. Set-up of a
+// product over 2.5x10^5 points with one lane / a warp / four lanes a cell: cells of 1.6 points 1.47 /
+// 2.55 / 1.34 ms, of 14 points 0.58 / 0.60 / 0.50 ms; of 100 points one lane 0.92, a warp 0.52 ms.
+static void launch_point_forms(const Grid& g0, const Grid* grids, const int* cprob, int ncell, const PointsView& p,
+                               const PointForms& o, cudaStream_t s) {
+  if (p.n < 16LL * ncell)
+    k_point_forms<4><<<ceil_div(ncell, 64), 256, 0, s>>>(g0, grids, cprob, ncell, p.cell_start, p.x, p.y, p.z, o);
+  else
+    k_point_forms<32><<<ceil_div(ncell, 8), 256, 0, s>>>(g0, grids, cprob, ncell, p.cell_start, p.x, p.y, p.z, o);
+  PRBF_CHECK_LAUNCH();
+}
+
 void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& src, unsigned* err,
                     Workspace& ws, cudaStream_t s, int forms) {
   (void)err;
@@ -1719,9 +1732,7 @@ void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& sr
     const bool f32 = forms & FORM_F32, fx = (forms & FORM_F64) && fx_grid_ok(g);
     if (f32 || fx) {
       const PointForms o = alloc_forms(plan, g.dim, src.n, f32, fx, s);
-      k_point_forms<<<ceil_div(g.ncell, 8), 256, 0, s>>>(g, nullptr, nullptr, g.ncell, src.cell_start, src.x, src.y,
-                                                         src.z, o);
-      PRBF_CHECK_LAUNCH();
+      launch_point_forms(g, nullptr, nullptr, g.ncell, src, o, s);
     }
     if (fx) {
       gauss_fx_upload_tables(s);
@@ -1732,9 +1743,7 @@ void gauss_plan_dev(GaussPlan& plan, const PointsView& tgt, const PointsView& sr
         PointForms ot;
         uint2** q[3] = {&ot.fx, &ot.fy, &ot.fz};
         for (int d = 0; d < g.dim; d++) *q[d] = plan.fxt[d].reserve(std::max(tgt.n, 1));
-        k_point_forms<<<ceil_div(g.ncell, 8), 256, 0, s>>>(g, nullptr, nullptr, g.ncell, tgt.cell_start, tgt.x, tgt.y,
-                                                           tgt.z, ot);
-        PRBF_CHECK_LAUNCH();
+        launch_point_forms(g, nullptr, nullptr, g.ncell, tgt, ot, s);
       }
     }
     plan.f32_ready = f32;
@@ -1847,9 +1856,7 @@ void gauss_plan_forms_batch(GaussPlan& plan, const std::vector<Grid>& grids, con
   const bool f32 = forms & FORM_F32;
   if (!f32 && !fx) return;
   const PointForms o = alloc_forms(plan, grids[0].dim, src.n, f32, fx, s);
-  k_point_forms<<<ceil_div(ncell, 8), 256, 0, s>>>(plan.g, plan.grids.get(), plan.cprob.get(), ncell, src.cell_start,
-                                                   src.x, src.y, src.z, o);
-  PRBF_CHECK_LAUNCH();
+  launch_point_forms(plan.g, plan.grids.get(), plan.cprob.get(), ncell, src, o, s);
   if (fx) gauss_fx_upload_tables(s);
   plan.fx_self = true;
   plan.fx_ncs = ncell + 1;
