@@ -130,8 +130,8 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
       if (it->second.stream) break;  // the same stream's first
     }
     if (best != r.second) {
+      P.used[best->second.p] = {d, cls};  // (may throw: *p is set last)
       *p = best->second.p;
-      P.used[*p] = {d, cls};
       D.cached -= cls;
       D.free.erase(best);
       return cudaSuccess;
@@ -149,6 +149,7 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
       P.used[*p] = {d, cls};
     } catch (const std::bad_alloc&) {
       cudaFree(*p);
+      *p = nullptr;
       throw;
     }
   }

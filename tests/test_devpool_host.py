@@ -132,13 +132,21 @@ int main() {
     CHECK(taken == t - 5 * MB);
     fail_new = true;
     bool thrown = false;
+    void *c = nullptr, *e = nullptr;
     try {
-      a = get(7 * MB);
+      dev_alloc(&c, 7 * MB);
+    } catch (const std::bad_alloc&) {
+      thrown = true;
+    }
+    CHECK(thrown && taken == t - 5 * MB && !c);
+    try {
+      thrown = false;
+      dev_alloc(&e, 6 * MB);  // (a kept block: stays kept)
     } catch (const std::bad_alloc&) {
       thrown = true;
     }
     fail_new = false;
-    CHECK(thrown && taken == t - 5 * MB);
+    CHECK(thrown && taken == t - 5 * MB && !e);
     CHECK(get(6 * MB) == b);
     dev_free(b);
   }
