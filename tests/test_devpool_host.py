@@ -33,7 +33,10 @@ cudaError_t cudaMalloc(void** p, size_t n) {
   if (taken + n > capacity) return cudaErrorMemoryAllocation;
   *p = next_address;
   next_address += (n + 511) / 512 * 512;
+  const bool f = fail_new;
+  fail_new = false;  // (the stand-in's own bookkeeping)
   live[*p] = n;
+  fail_new = f;
   taken += n;
   return cudaSuccess;
 }
